@@ -28,7 +28,8 @@ HOST_SOURCES = ["lang/yaml.cpp", "lang/lang.cpp", "lang/codegen.cpp", "runtime/j
                 "runtime/engine.cpp", "runtime/batch.cpp", "runtime/server.cpp", "runtime/snapshot.cpp",
                 "capi.cpp"]
 CUDA_SOURCES = ["kernels/devutil.cu", "kernels/render.cu"]
-EMBED = [("SE_PRELUDE_SRC", "kernels/prelude.cuh"), ("SE_MARGOLUS_SRC", "kernels/margolus.cuh")]
+EMBED = [("SE_PRELUDE_SRC", "kernels/prelude.cuh"), ("SE_MARGOLUS_SRC", "kernels/margolus.cuh"),
+         ("SE_NIBBLE_SRC", "kernels/nibble.cuh")]
 
 
 def _embed_header() -> str:

@@ -677,6 +677,53 @@ __device__ __forceinline__ void se_tile_edits(uint8_t* sm, int SW, int SH, int g
   }
 }
 
+// Rule sets with a block transition table of 4-bit keys run their multi-frame tiles with two
+// cells per byte (nibble.cuh), unless their rules compare hash values besides the mirror test and use
+// all 16 ids (SE_NIB needs id 15 to mark blocks).
+#if defined(SE_LUT)
+#if SE_LUT_BITS == 4 && (SE_NMAT <= 15 || SE_LUT_ENTRIES <= 2u * SE_LUT_KEYS)
+#define SE_NIB 1
+#endif
+#endif
+
+#ifdef SE_NIB
+// After the full table and its static bits: the reduced table, the static-material mask and,
+// with hash comparisons besides the mirror test, the bound table (se_build_nib).
+#define SE_NIB_OFF ((SE_LUT_STATIC_OFF + SE_LUT_STATIC_WORDS * 4u + 15u) & ~15u)
+#define SE_NIB_CLASSES (SE_LUT_ENTRIES / SE_LUT_KEYS)
+// Hash comparisons besides the mirror test: SE_NIB_PROB; SE_NIB_LANE is the one lane they
+// read, or 0 when they read several (or lane 0).
+#define SE_NIB_PROB (SE_NIB_CLASSES > 2u)
+#if SE_LUT_N0 == 2u && SE_LUT_N1 == SE_NIB_CLASSES / 2u
+#define SE_NIB_LANE 1
+#define SE_NIB_MUL 2131u
+#elif SE_LUT_N0 == 2u && SE_LUT_N2 == SE_NIB_CLASSES / 2u
+#define SE_NIB_LANE 2
+#define SE_NIB_MUL 21313u
+#elif SE_LUT_N0 == 2u && SE_LUT_N3 == SE_NIB_CLASSES / 2u
+#define SE_NIB_LANE 3
+#define SE_NIB_MUL 213132u
+#else
+#define SE_NIB_LANE 0
+#endif
+// Up to 8 materials the reduced table (at most 16 KB) is indexed in radix SE_NMAT and copied
+// into shared memory: random lookups conflict on a few banks there, where a gather through
+// L1 takes a pass per 128-byte line.  Beyond that it is indexed by the 4-bit ids and read
+// through the read-only cache.
+#define SE_NIB_SHARED (SE_NMAT <= 8)
+#define SE_NIB_ENTRIES (SE_NIB_SHARED ? SE_NMAT * SE_NMAT * SE_NMAT * SE_NMAT : 65536)
+#define SE_NIB_BOUNDS ((SE_NIB_ENTRIES + 2) & ~1)  // the bound table's first word
+// Launch bounds of the multi-frame tile kernels: up to 64 registers, for eight lookups and eight hashes of
+// a lane in flight (32 warps an SM; 40 or 48 at 48 or 40 registers ran 1% and 5% slower).
+#define SE_TILE_BOUNDS(NT) __launch_bounds__(NT, 1024 / NT)
+template <int TW, int TH, int KMAX, int NT>
+__device__ __forceinline__ void se_nib_run(const uint32_t* __restrict__ src, uint32_t* __restrict__ dst, int W,
+                                           int H, int f0, int k, const uint16_t* __restrict__ lut, int X0, int Y0,
+                                           int ya, int yb, const SeEditParams* __restrict__ edits, int nedits);
+#else
+#define SE_TILE_BOUNDS(NT) __launch_bounds__(NT)
+#endif
+
 // Advances the tile with top-left cell (X0, Y0) of a W x H world by k <= KMAX frames whose
 // counters are f0, f0+1, ... (all >= 2; the host handles the frame-1 clear).
 // src and dst hold the world rows [ya, yb) (row gy at (gy - ya) * W): the whole world, or a
@@ -689,6 +736,14 @@ __device__ __forceinline__ void se_tile_run(const uint32_t* __restrict__ src, ui
                                             int H, int f0, int k, const uint16_t* __restrict__ lut, int X0, int Y0,
                                             int ya, int yb, const SeEditParams* __restrict__ edits = nullptr,
                                             int nedits = 0) {
+#ifdef SE_NIB
+  // One-frame launches keep byte tiles: they run at the memory's speed, and packing the cells
+  // costs more than it saves there (85 against 108 us a frame of an 8192 x 8192 world).
+  if constexpr (KMAX > 1) {
+    se_nib_run<TW, TH, KMAX, NT>(src, dst, W, H, f0, k, lut, X0, Y0, ya, yb, edits, nedits);
+    return;
+  }
+#endif
   constexpr int HX = ((KMAX + 3) / 4) * 4, HY = KMAX;
   constexpr int SW = TW + 2 * HX, SH = TH + 2 * HY, WPR = SW / 4;
   static_assert(TW % 4 == 0, "tile width must be a multiple of 4");

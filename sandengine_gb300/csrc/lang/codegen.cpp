@@ -1101,6 +1101,8 @@ bool generate_cuda(const ParsingResult& r, CudaRules* out, ParseError* err) {
       o << "#define SE_LUT 1\n#define SE_LUT_BITS " << bits << "\n#define SE_LUT_ENTRIES " << entries << "u\n"
         << "#define SE_LUT_KEYS " << keys << "u\n#define SE_LUT_STATIC_WORDS " << std::max<uint64_t>(1, keys / 32)
         << "u\n";
+      // Hash classes per lane; entries are numbered key, lane 0's class, ..., lane 3's class.
+      for (int l = 0; l < 4; ++l) o << "#define SE_LUT_N" << l << " " << g.bounds[l].size() + 1 << "u\n";
       // The key of the block [a b / c d] (top-left, top-right, bottom-left, bottom-right) in
       // column order, a | c << bits | b << 2 bits | d << 3 bits: with 4 bits, a row pair's
       // two keys are its top row word plus its bottom row word << 4 (se_chunk_eval).

@@ -236,7 +236,7 @@ Status Batch::autotune(int reps, int* best_k) {
   const TileVariant* best = nullptr;
   if (tiled.empty()) {
     for (const TileVariant& v : tile_variants())
-      if (!best || v.kmax > best->kmax) best = &v;  // only the pass count matters
+      if (v.fits(rs->lut_shape()) && (!best || v.kmax > best->kmax)) best = &v;  // only the pass count matters
   } else {
     cudaEvent_t a, b;
     SE_CUDA(cudaEventCreate(&a));
@@ -245,6 +245,7 @@ Status Batch::autotune(int reps, int* best_k) {
     for (int w : tiled) tiled_cells += (long long)desc[(size_t)w].W * desc[(size_t)w].H;
     double best_rate = 0;
     for (const TileVariant& v : tile_variants()) {
+      if (!v.fits(rs->lut_shape())) continue;
       Status s = set_variant(&v);
       if (!s.ok()) return s;
       const size_t smem = tile_smem_bytes(v, rs->lut_shape());
@@ -302,10 +303,7 @@ Status Batch::step(int F) {
     Status s = steps_per_launch > 0 ? Status::Ok() : autotune(2, nullptr);
     if (!s.ok()) return s;
     if (!variant) {
-      const TileVariant* v = nullptr;
-      for (const TileVariant& t : tile_variants())
-        if (t.kmax >= steps_per_launch && (!v || t.kmax < v->kmax)) v = &t;
-      s = set_variant(v);
+      s = set_variant(pick_variant(steps_per_launch, rs->lut_shape()));
       if (!s.ok()) return s;
     }
   }
@@ -335,12 +333,7 @@ Status Batch::step(int F) {
 
 Status Batch::step_plain(int F) {
   if (F < 0) return {SE_ERR_INVALID_ARGUMENT, "nframes must be >= 0"};
-  const TileVariant* v1 = nullptr;
-  for (const TileVariant& t : tile_variants())
-    if (t.kmax == 1) {
-      v1 = &t;
-      break;
-    }
+  const TileVariant* v1 = pick_variant(1, rs->lut_shape());
   for (int f = 0; f < F; ++f) {
     for (auto& d : desc) {
       const int fr = d.frame + 1;

@@ -57,13 +57,17 @@ Status Ruleset::ensure_loaded() {
   if (!m->load(cubin, lut_shape(), &err)) return {SE_ERR_CUDA, err};
   if (cuda.lut_entries) {  // build the block transition table with the rules themselves
     const size_t table = ((size_t)cuda.lut_entries * sizeof(uint16_t) + 15) & ~(size_t)15;
-    cudaError_t e = cudaMalloc(&d_lut, table + (size_t)cuda.lut_static_words * 4);
+    const size_t nib_off = (table + (size_t)cuda.lut_static_words * 4 + 15) & ~(size_t)15;  // SE_NIB_OFF
+    const unsigned long long nib = lut_shape().nib_words;
+    cudaError_t e = cudaMalloc(&d_lut, nib_off + nib * 4);
     if (e != cudaSuccess) return {SE_ERR_OUT_OF_MEMORY, std::string("cudaMalloc: ") + cudaGetErrorString(e)};
     void* args[] = {(void*)&d_lut};
     const unsigned blocks = (unsigned)std::min<unsigned long long>((cuda.lut_entries + 255) / 256, 4096);
     SE_CUDA(cudaLaunchKernel((const void*)m->get("se_build_lut"), dim3(blocks), dim3(256), args, 0, nullptr));
     const unsigned sblocks = (unsigned)((cuda.lut_static_words + 255) / 256);
     SE_CUDA(cudaLaunchKernel((const void*)m->get("se_build_static"), dim3(sblocks), dim3(256), args, 0, nullptr));
+    if (nib)
+      SE_CUDA(cudaLaunchKernel((const void*)m->get("se_build_nib"), dim3(256), dim3(256), args, 0, nullptr));
     SE_CUDA(cudaDeviceSynchronize());
   }
   {  // render table (operations.glsl:68-70, 100-108, 126): colour, emission and flags
@@ -170,13 +174,6 @@ int World::default_k() const {
   return fused ? fused->kmax : 1;
 }
 
-static const TileVariant* pick_variant(int k) {
-  const TileVariant* best = nullptr;
-  for (const TileVariant& t : tile_variants())
-    if (t.kmax >= k && (!best || t.kmax < best->kmax)) best = &t;
-  return best;
-}
-
 Status World::autotune(int reps, int* best_k) {
   TraceRange trace("se_world_autotune");
   if (reps < 1) reps = 1;
@@ -193,6 +190,7 @@ Status World::autotune(int reps, int* best_k) {
   double best_multi = 0, best_one = 0;
   const TileVariant *vm = nullptr, *v1 = nullptr;
   for (const TileVariant& v : tile_variants()) {
+    if (!v.fits(rs->lut_shape())) continue;
     Status s = launch_tiles(f0, v.kmax, &v, false);  // warm-up
     if (!s.ok()) return s;
     SE_CUDA(cudaEventRecord(a, stream));
@@ -371,15 +369,15 @@ Status World::step(int nframes, const se_modification* mods, int nmods) {
   while (nlive < nseen && mods[nlive].mod_size != 0) ++nlive;  // falling_sand.glsl:139-141
   const TileVariant* vmulti = nullptr;
   if (steps_per_launch > 0) {
-    vmulti = pick_variant(steps_per_launch);
+    vmulti = pick_variant(steps_per_launch, rs->lut_shape());
   } else {
     if (!fused && nframes >= 2) {
       Status s = autotune(2, nullptr);
       if (!s.ok()) return s;
     }
-    vmulti = fused ? fused : pick_variant(1);
+    vmulti = fused ? fused : pick_variant(1, rs->lut_shape());
   }
-  const TileVariant* vone = single ? single : pick_variant(1);
+  const TileVariant* vone = single ? single : pick_variant(1, rs->lut_shape());
   const int kdef = steps_per_launch > 0 ? steps_per_launch : vmulti->kmax;
   if (light[0]) {  // one frame at a time, each followed by the light pass
     for (int i = 0; i < nframes; ++i) {

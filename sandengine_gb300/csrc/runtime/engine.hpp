@@ -44,7 +44,19 @@ struct Ruleset {
   // Per-material colour / emission / flags for the colour and light passes.
   RenderMat* d_render = nullptr;
   ~Ruleset();
-  LutShape lut_shape() const { return {cuda.lut_entries, cuda.lut_static_words}; }
+  LutShape lut_shape() const {
+    LutShape s;
+    s.entries = cuda.lut_entries;
+    s.static_words = cuda.lut_static_words;
+    const unsigned long long n = (unsigned long long)num_materials(), keys = 65536;
+    const bool prob = s.entries > 2 * keys;
+    if (s.entries && s.static_words == keys / 32 && (n <= 15 || !prob)) {  // SE_NIB in the kernels
+      s.nib_shared = n <= 8;
+      s.nib_entries = s.nib_shared ? n * n * n * n : keys;
+      s.nib_words = ((s.nib_entries + 2) & ~1ull) + (prob ? 2 * keys : 0);  // SE_NIB_BOUNDS
+    }
+    return s;
+  }
   // CHECKED build: the module is compiled with SE_CHECKED (index checks recorded in the
   // device word se_check_word); set before the first compile.
   bool checked = false;

@@ -11,7 +11,7 @@
 #include <mutex>
 #include <sstream>
 
-#include "kernel_src.inc"  // SE_PRELUDE_SRC, SE_MARGOLUS_SRC (generated from csrc/kernels)
+#include "kernel_src.inc"  // SE_PRELUDE_SRC, SE_MARGOLUS_SRC, SE_NIBBLE_SRC (generated from csrc/kernels)
 
 namespace se::rt {
 
@@ -24,41 +24,55 @@ std::string TileVariant::edit_name() const {
 }
 
 // Tile shapes and fusion depths compiled into every rule-set module; the launcher and the
-// autotuner choose among them.  Larger tiles recompute a smaller share of halo cells per
-// fused step (128x64 at k=8: 1.41x the tile's cells; 256x128 at k=8: 1.20x).  The shared
-// array must stay under 65,536 cells (16-bit offsets in the chunk list).
+// autotuner choose among those marked for the rule set's kind of tile.  Larger tiles
+// recompute a smaller share of halo cells per fused step (128x64 at k=8: 1.41x the tile's
+// cells; 256x128 at k=8: 1.20x; 240x240: 1.14x).  Byte tiles must stay under 65,536 cells
+// (16-bit offsets in the chunk list).  The arrays of 4-bit tiles take whole warp items of
+// 32 x 32 cells, tile and halo together, so their shapes are 32 n - 2 halo.
 const std::vector<TileVariant>& tile_variants() {
+  constexpr int B = TileVariant::kByte, N = TileVariant::kNibble;
   static const std::vector<TileVariant> v = {
-      {128, 64, 1, 256},  {256, 32, 1, 256},  {128, 32, 1, 256},  {128, 64, 2, 256},
-      {128, 64, 4, 256},  {128, 64, 8, 256},  {128, 128, 8, 256}, {128, 128, 16, 256},
-      {256, 64, 4, 256},  {64, 64, 4, 256},   {256, 128, 8, 512}, {192, 128, 8, 256},
-      {256, 128, 4, 512}, {256, 64, 8, 256},
+      {128, 64, 1, 256, B | N}, {256, 32, 1, 256, B | N}, {128, 32, 1, 256, B | N}, {128, 64, 2, 256, B},
+      {128, 64, 4, 256, B},     {128, 64, 8, 256, B},     {128, 128, 8, 256, B},    {128, 128, 16, 256, B},
+      {256, 64, 4, 256, B},     {64, 64, 4, 256, B},      {256, 128, 8, 512, B},    {192, 128, 8, 256, B},
+      {256, 128, 4, 512, B},    {256, 64, 8, 256, B},
+      {120, 120, 4, 128, N},    {56, 56, 4, 128, N},      {112, 112, 8, 128, N},    {112, 48, 8, 128, N},
+      {48, 48, 8, 128, N},      {240, 176, 8, 256, N},    {240, 240, 8, 256, N},    {96, 96, 16, 128, N},
   };
   return v;
 }
 
+const TileVariant* pick_variant(int k, const LutShape& lut) {
+  const TileVariant* best = nullptr;
+  for (const TileVariant& t : tile_variants())
+    if (t.kmax >= k && t.fits(lut) && (!best || t.kmax < best->kmax)) best = &t;
+  return best;
+}
+
 std::string kernel_source(const std::string& generated_rules) {
   std::ostringstream o;
-  o << SE_PRELUDE_SRC << "\n" << generated_rules << "\n" << SE_MARGOLUS_SRC << "\n";
+  o << SE_PRELUDE_SRC << "\n" << generated_rules << "\n" << SE_MARGOLUS_SRC << "\n"
+    << SE_NIBBLE_SRC << "\n";
   for (const TileVariant& t : tile_variants()) {
-    o << "extern \"C\" __global__ void __launch_bounds__(" << t.nt << ") " << t.name()
+    const std::string bounds = (t.kmax > 1 ? "SE_TILE_BOUNDS(" : "__launch_bounds__(") + std::to_string(t.nt) + ") ";
+    o << "extern \"C\" __global__ void " << bounds << t.name()
       << "(const uint32_t* __restrict__ src, uint32_t* __restrict__ dst, int W, int H, int f0, int k,"
          " const uint16_t* __restrict__ lut, int ya, int yb) {\n"
       << "  se_tile_impl<" << t.tw << ", " << t.th << ", " << t.kmax << ", " << t.nt
       << ">(src, dst, W, H, f0, k, lut, ya, yb);\n}\n";
     // the edit list travels in the parameter space, read in place (__grid_constant__)
-    o << "extern \"C\" __global__ void __launch_bounds__(" << t.nt << ") " << t.edit_name()
+    o << "extern \"C\" __global__ void " << bounds << t.edit_name()
       << "(const uint32_t* __restrict__ src, uint32_t* __restrict__ dst, int W, int H, int f0, int k,"
          " const uint16_t* __restrict__ lut, int ya, int yb, const __grid_constant__ SeEditParams edits,"
          " int nedits) {\n"
       << "  se_tile_impl<" << t.tw << ", " << t.th << ", " << t.kmax << ", " << t.nt
       << ">(src, dst, W, H, f0, k, lut, ya, yb, &edits, nedits);\n}\n";
-    o << "extern \"C\" __global__ void __launch_bounds__(" << t.nt << ") " << t.multi_name()
+    o << "extern \"C\" __global__ void " << bounds << t.multi_name()
       << "(const SeWorldDesc* __restrict__ worlds, const SeTileJob* __restrict__ jobs, int pass,"
          " int frames_done, int k, const uint16_t* __restrict__ lut) {\n"
       << "  se_mtile_impl<" << t.tw << ", " << t.th << ", " << t.kmax << ", " << t.nt
       << ">(worlds, jobs, pass, frames_done, k, lut);\n}\n";
-    o << "extern \"C\" __global__ void __launch_bounds__(" << t.nt << ") " << t.serve_name()
+    o << "extern \"C\" __global__ void " << bounds << t.serve_name()
       << "(const SeWorldDesc* __restrict__ descs, const int* __restrict__ prefix, int nactive,"
          " const uint16_t* __restrict__ lut) {\n"
       << "  se_stile_impl<" << t.tw << ", " << t.th << ", " << t.kmax << ", " << t.nt
@@ -170,7 +184,12 @@ Module::~Module() {
 }
 
 size_t tile_smem_bytes(const TileVariant& t, const LutShape& lut) {
-  (void)lut;
+  if (lut.nib_entries && t.kmax > 1) {  // SeNib's array (nibble.cuh) and, when small, its reduced table
+    const size_t sw16 = (size_t)(t.sw() + 15) / 16, wpr = 2 * ((sw16 + 1) / 2 * 2);
+    const size_t stride = wpr + (wpr % 4 == 0 ? 2 : 4);
+    const size_t rows = 32 * (((size_t)(t.sh() + 1) / 2 + 15) / 16) + 1;
+    return (((stride * rows + 3) & ~(size_t)3) + (lut.nib_shared ? lut.nib_entries : 0)) * 4;
+  }
   size_t b = (t.smem_bytes() + 15) & ~(size_t)15;
   // 48-byte header (slack, list counters, uniform-material flags), then the per-step list
   // of chunks (4 blocks) to evaluate, one u16 offset each
@@ -190,6 +209,7 @@ bool Module::load(const std::string& cubin, const LutShape& lut, std::string* er
     names.push_back("se_build_lut");
     names.push_back("se_build_static");
   }
+  if (lut.nib_entries) names.push_back("se_build_nib");
   for (auto& t : tile_variants()) {
     names.push_back(t.name());
     names.push_back(t.edit_name());

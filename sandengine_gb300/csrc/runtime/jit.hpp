@@ -10,9 +10,23 @@
 
 namespace se::rt {
 
+// Size of a rule set's block transition table: its u16 entries and the 32-bit words of the
+// bitset of static keys that follows it (both 0 without a table).
+struct LutShape {
+  unsigned long long entries = 0, static_words = 0;
+  // Rule sets whose tiles pack two cells a byte (nibble.cuh): the entries of the reduced table
+  // (0: byte tiles), whether each CTA copies it into shared memory, and the 32-bit words of
+  // all that follows the static bits.
+  unsigned long long nib_entries = 0, nib_words = 0;
+  bool nib_shared = false;
+};
+
 // A tile-kernel instantiation: TW x TH output cells, up to KMAX frames per launch.
 struct TileVariant {
   int tw, th, kmax, nt;
+  enum { kByte = 1, kNibble = 2 };
+  int use;  // the kinds of tile it is chosen for (set_tile may ask for any)
+  bool fits(const LutShape& lut) const { return use & (lut.nib_entries ? kNibble : kByte); }
   std::string name() const;        // single-world kernel
   std::string edit_name() const;   // single-world kernel with the first frame's edit pass
   std::string multi_name() const;  // many-world (tile job list) kernel
@@ -24,15 +38,13 @@ struct TileVariant {
   size_t smem_bytes() const { return (size_t)sw() * (size_t)sh(); }
 };
 const std::vector<TileVariant>& tile_variants();
+// The variant for k frames per launch: of those chosen for the rule set's tiles the first with
+// the fewest frames >= k.
+const TileVariant* pick_variant(int k, const LutShape& lut);
 
-// Size of a rule set's block transition table: its u16 entries and the 32-bit words of the
-// bitset of static keys that follows it (both 0 without a table).
-struct LutShape {
-  unsigned long long entries = 0, static_words = 0;
-};
 // Dynamic shared memory of a tile launch: the u8 tile, then the per-step list of chunks to
-// evaluate.  The block transition table and its static-key bitset stay in global memory
-// (read through the read-only cache).
+// evaluate; or the 4-bit tile and a small reduced table.  The block transition table and its
+// static-key bitset stay in global memory (read through the read-only cache).
 size_t tile_smem_bytes(const TileVariant& t, const LutShape& lut);
 
 // Full device source: prelude + generated rules + kernel template + instantiations.

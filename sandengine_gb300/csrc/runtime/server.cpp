@@ -74,9 +74,7 @@ Status Server::set_frames_per_iteration(int k) {
   // throughput, 770 G cell-updates/s, against 690-734 G with 256x128, 128x128 or 256x64
   // tiles): their smaller halo loss on the large tiles does not make up for the waste on
   // the small sessions and the coarser work units of an iteration.
-  const TileVariant* v = nullptr;
-  for (const TileVariant& t : tile_variants())
-    if (t.kmax >= k && (!v || t.kmax < v->kmax)) v = &t;
+  const TileVariant* v = pick_variant(k, rs->lut_shape());
   if (!v || k < 1) return {SE_ERR_INVALID_ARGUMENT, "no kernel variant for this many frames per iteration"};
   variant = v;
   return Status::Ok();
@@ -610,12 +608,7 @@ Status Server::serve_plain(std::unique_lock<std::mutex>& lk) {
     std::stable_sort(pend.begin(), pend.end(),
                      [&](int a, int b) { return requests[(size_t)a].arrival_ms < requests[(size_t)b].arrival_ms; });
   }
-  const TileVariant* v1 = nullptr;
-  for (const TileVariant& t : tile_variants())
-    if (t.kmax == 1) {
-      v1 = &t;
-      break;
-    }
+  const TileVariant* v1 = pick_variant(1, rs->lut_shape());
   size_t next = 0;
   for (;;) {
     int ri = -1;
