@@ -1073,6 +1073,10 @@ __device__ __forceinline__ void se_rt_step(uint8_t* sm, int SW, int SH, int ly0,
   }
 }
 
+#ifdef SE_NIB
+__device__ __forceinline__ void se_nib_resident(const SeWorldDesc& w, int frames, int out_flip,
+                                                const uint16_t* __restrict__ lut);
+#endif
 // Whole-world launch: CTA b holds world ids[b] entirely in shared memory (plus a WALL
 // border: 4 columns on the left and at least 4 on the right, the row stride a multiple of
 // 8; 1 row above and below), advances it by `frames` frames and stores it to the buffer
@@ -1083,8 +1087,11 @@ __device__ __forceinline__ void se_rt_step(uint8_t* sm, int SW, int SH, int ly0,
 extern "C" __global__ void __launch_bounds__(1024) se_resident(const SeWorldDesc* __restrict__ worlds,
                                                                const int* __restrict__ ids, int frames, int out_flip,
                                                                const uint16_t* __restrict__ lut) {
-  extern __shared__ __align__(16) uint8_t se_smem[];
   const SeWorldDesc w = worlds[ids[blockIdx.x]];
+#ifdef SE_NIB
+  se_nib_resident(w, frames, out_flip, lut);
+#else
+  extern __shared__ __align__(16) uint8_t se_smem[];
   const int SW = ((w.W + 7) & ~7) + 8, SH = w.H + 2;
   const int gx0 = -4, gy0 = -1;
   const int HDR = (SW * SH + 15) & ~15, cap = (SW / 8) * (SH / 2);
@@ -1111,6 +1118,7 @@ extern "C" __global__ void __launch_bounds__(1024) se_resident(const SeWorldDesc
     __syncthreads();
   }
   se_store_region(se_smem, SW, 4, 1, w.W, w.H, dst, w.W, w.H, 0, 0, blockDim.x);
+#endif
 }
 
 // After a launch of `frames` frames in `passes` passes: advance every world's counter and

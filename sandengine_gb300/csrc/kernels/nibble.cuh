@@ -508,4 +508,97 @@ __device__ __forceinline__ void se_nib_run(const uint32_t* __restrict__ src, uin
     }
   }
 }
+
+// One frame of a whole world (se_nib_resident's array): chunk i of cpr * nby, a lane each.
+template <int OX>
+__device__ __forceinline__ void se_nib_world_step(uint32_t* sm, int stride, int rows, int cpr, float inv_cpr, bool& look,
+                                                  int ly0, int gx0, int gy0, int f, int W, int H, uint32_t umask,
+                                                  const uint32_t* tab, const uint32_t* __restrict__ gtab,
+                                                  const uint16_t* __restrict__ lut) {
+#if defined(__CUDA_ARCH__)
+  constexpr int NT = 32;
+#else
+  constexpr int NT = 1;  // emulated: one thread per CTA
+#endif
+  const int lane = threadIdx.x & (NT - 1), nc = cpr * ((rows - ly0) / 2);
+  int still = 0, seen = 0;
+  for (int base = threadIdx.x & ~(NT - 1); base < nc; base += blockDim.x) {  // warp-uniform trip count
+    const bool on = base + lane < nc;
+    int j, q;
+    se_divmod_rt(on ? base + lane : base, cpr, inv_cpr, j, q);
+    const int row = ly0 + 2 * j, off = row * stride + 2 * q, gx = gx0 + 16 * q + OX, gy = gy0 + row;
+    if (!se_check(off >= 0 && off + stride + 2 < stride * rows, 8u)) break;
+    if (look) ++seen;
+    const uint32_t x = (uint32_t)gx * 461u + (uint32_t)gy * 2131u + (uint32_t)f * 4541161u;
+    if (se_nib_chunk<NT, OX>(sm, off, stride, on, look, gx, gy, x, W, H, true, umask, tab, gtab, lut)) ++still;
+  }
+  look = 8 * still > seen;
+}
+
+// se_resident's body on a word-packed array: the whole world with a WALL border of 4 columns on
+// the left, at least one on the right, and one row above and below; two words of padding per
+// row.  A world takes half a byte a cell, so worlds of up to about 450,000 cells fit a CTA.
+__device__ __forceinline__ void se_nib_resident(const SeWorldDesc& w, int frames, int out_flip,
+                                                const uint16_t* __restrict__ lut) {
+  extern __shared__ __align__(16) uint8_t se_smem[];
+  const int W = w.W, H = w.H, cpr = (W + 5 + 15) / 16, stride = 2 * cpr + 2, rows = H + 2, nt = blockDim.x;
+  uint32_t* sm = reinterpret_cast<uint32_t*>(se_smem);
+  const uint32_t* gtab = reinterpret_cast<const uint32_t*>(reinterpret_cast<const uint8_t*>(lut) + SE_NIB_OFF);
+  uint32_t* tab = sm + ((stride * rows + 3) & ~3);
+#if defined(__CUDA_ARCH__)
+  const uint32_t umask = __ldg(gtab + SE_NIB_ENTRIES);
+#if SE_NIB_SHARED
+  for (int i = threadIdx.x; i < SE_NIB_ENTRIES; i += nt) tab[i] = __ldg(gtab + i);
+#endif
+#else
+  const uint32_t umask = se_nib_static_mask(lut);
+#endif
+  for (int i = threadIdx.x; i < stride * rows; i += nt) sm[i] = 0x22222222u;
+  __syncthreads();
+  const uint32_t* src = w.cur ? w.buf1 : w.buf0;
+  uint32_t* dst = (w.cur ^ out_flip) ? w.buf1 : w.buf0;
+  uint16_t* sh = reinterpret_cast<uint16_t*>(se_smem);
+  const int hpr = (W + 3) / 4;  // half-words (four cells) of world cells per row
+  const float inv_hpr = 1.0f / (float)hpr, inv_cpr = 1.0f / (float)cpr;
+  const bool vec = (W & 3) == 0;
+  for (int i = threadIdx.x; i < hpr * H; i += nt) {
+    int y, c;
+    se_divmod_rt(i, hpr, inv_hpr, y, c);
+    const uint32_t* p = src + (size_t)y * W + 4 * c;
+    uint4 v;
+    if (vec) {
+      v = __ldg(reinterpret_cast<const uint4*>(p));
+    } else {
+      v.x = __ldg(p);
+      v.y = 4 * c + 1 < W ? __ldg(p + 1) : SE_WALL;
+      v.z = 4 * c + 2 < W ? __ldg(p + 2) : SE_WALL;
+      v.w = 4 * c + 3 < W ? __ldg(p + 3) : SE_WALL;
+    }
+    const int k = (y + 1) * 2 * stride + 1 + c;
+    if (se_check(k < 2 * stride * rows, 2u)) sh[k] = (uint16_t)se_nib_pack(v);
+  }
+  __syncthreads();
+  bool look = true;
+  for (int s = 0; s < frames; ++s) {
+    const int f = w.frame + 1 + s, ly0 = (se_off_y(f) - 1) & 1;
+    if (se_off_x(f) == 0)
+      se_nib_world_step<0>(sm, stride, rows, cpr, inv_cpr, look, ly0, -4, -1, f, W, H, umask, tab, gtab, lut);
+    else
+      se_nib_world_step<1>(sm, stride, rows, cpr, inv_cpr, look, ly0, -4, -1, f, W, H, umask, tab, gtab, lut);
+    if ((s & 63) == 63) look = true;  // the world may have come to rest
+    __syncthreads();
+  }
+  for (int i = threadIdx.x; i < hpr * H; i += nt) {
+    int y, c;
+    se_divmod_rt(i, hpr, inv_hpr, y, c);
+    const uint32_t h = sh[(y + 1) * 2 * stride + 1 + c];
+    uint32_t* p = dst + (size_t)y * W + 4 * c;
+    if (vec) {
+      *reinterpret_cast<uint4*>(p) = make_uint4(h & 15u, (h >> 4) & 15u, (h >> 8) & 15u, h >> 12);
+    } else {
+      for (int e = 0; e < 4; ++e)
+        if (4 * c + e < W) p[e] = (h >> (4 * e)) & 15u;
+    }
+  }
+}
 #endif  // SE_NIB

@@ -19,10 +19,14 @@ Status cuda_fail(const char* what, cudaError_t e) {
     if (_e != cudaSuccess) return cuda_fail(#call, _e); \
   } while (0)
 
-// Shared memory of a whole world in se_resident: the array (row stride a multiple of 8, a
-// WALL border), a 48-byte header and a chunk list of one u16 entry per chunk.
+// Shared memory of a whole world in se_resident: with 4-bit tiles se_nib_resident's array and
+// a small reduced table; else the byte array (row stride a multiple of 8, a WALL border), a
+// 48-byte header and a chunk list of one u16 entry per chunk.
 size_t resident_bytes(int W, int H, const LutShape& lut) {
-  (void)lut;
+  if (lut.nib_entries) {
+    const size_t stride = 2 * (((size_t)W + 5 + 15) / 16) + 2, rows = (size_t)H + 2;
+    return (((stride * rows + 3) & ~(size_t)3) + (lut.nib_shared ? lut.nib_entries : 0)) * 4;
+  }
   const size_t SW = (size_t)(((W + 7) & ~7) + 8), SH = (size_t)H + 2;
   const size_t cap = (SW / 8) * (SH / 2);
   return ((SW * SH + 15) & ~(size_t)15) + 48 + ((2 * cap + 15) & ~(size_t)15);
@@ -92,18 +96,33 @@ Status Batch::create(std::shared_ptr<Ruleset> r, int count, const int* widths, c
 Status Batch::classify() {
   const size_t maxsm = rs->module->max_dyn_smem;
   const LutShape lut = rs->lut_shape();
-  // size classes for whole-world CTAs: occupancy is set by the largest world of a class
-  const size_t class_max[3] = {40 * 1024, 100 * 1024, maxsm};
-  const int class_threads[3] = {256, 512, 1024};
+  // Size classes for whole-world CTAs: occupancy is set by the largest world of a class.  A
+  // 4-bit world has one chunk of 16 x 2 cells per 16 bytes: two to eight chunks a lane.
+  const bool nib = lut.nib_entries > 0;
+  const size_t table = nib && lut.nib_shared ? lut.nib_entries * 4 : 0;
+  const size_t class_max[4] = {nib ? table + 8 * 1024 : 40 * 1024, nib ? table + 32 * 1024 : 100 * 1024,
+                               nib ? table + 72 * 1024 : maxsm, maxsm};
+  const int class_threads[4] = {nib ? 128 : 256, 512, nib ? 768 : 1024, 1024};
+  // A whole-world CTA is one SM's work from start to end: in a batch of few worlds a large one
+  // would still run when the others are done, and is better spread over the SMs as tiles
+  // (unless the caller set the limit).  The line lies at half an SM's share of the cells, and
+  // at 20,000 cells (200 frames, twelve materials; lines at 0.25 / 0.5 / 1 / 2 shares: 150
+  // worlds of 64-1024 cells a side 2.87 / 2.79 / 2.82 / 2.90 ms, 300 worlds 4.35 / 4.34 / 4.63
+  // / 5.80 ms, 1000 worlds 11.2 / 10.0 / 9.9 / 9.9 ms; 20 worlds of 64-512 with the floor at
+  // 20,000 / 50,000 / 100,000 cells 0.39 / 0.67 / 0.94 ms).
+  int dev = 0, sms = 0;
+  SE_CUDA(cudaGetDevice(&dev));
+  SE_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+  const long long fair = nib && !limit_set ? std::max<long long>(20000, cells / (2 * std::max(sms, 1))) : LLONG_MAX;
   for (auto& R : resident)
     if (R.d_ids) cudaFree(R.d_ids);
-  resident.assign(3, Resident{});
+  resident.assign(4, Resident{});
   tiled.clear();
   for (int i = 0; i < n; ++i) {
     const size_t rb = resident_bytes(desc[(size_t)i].W, desc[(size_t)i].H, lut);
     int cls = -1;
-    if (rb <= resident_limit)
-      for (int c = 0; c < 3; ++c)
+    if (rb <= resident_limit && (long long)desc[(size_t)i].W * desc[(size_t)i].H <= fair)
+      for (int c = 0; c < 4; ++c)
         if (rb <= class_max[c]) {
           cls = c;
           break;
@@ -111,7 +130,7 @@ Status Batch::classify() {
     if (cls < 0) tiled.push_back(i);
     else resident[(size_t)cls].ids.push_back(i);
   }
-  for (int c = 0; c < 3; ++c) {
+  for (int c = 0; c < 4; ++c) {
     Resident& R = resident[(size_t)c];
     R.threads = class_threads[c];
     std::sort(R.ids.begin(), R.ids.end(), [&](int a, int b) {
@@ -129,6 +148,7 @@ Status Batch::classify() {
 
 Status Batch::set_resident_limit(size_t bytes) {
   resident_limit = bytes;
+  limit_set = true;
   Status s = classify();
   if (!s.ok()) return s;
   if (variant) return set_variant(variant);  // the tile job list

@@ -64,6 +64,7 @@ struct Batch {
   // others take tile passes (0: none resident).  Rebuilds the classes and the job list.
   Status set_resident_limit(size_t bytes);
   size_t resident_limit = 0;
+  bool limit_set = false;  // by set_resident_limit
 
  private:
   Status classify();
