@@ -10,7 +10,7 @@ namespace se::rt {
 
 // One material's render data.  Ids >= the table size read entry 1 (NULL), as
 // getMaterialFromID returns MAT_NULL for unknown ids.
-struct RenderMat {
+struct alignas(16) RenderMat {
   float color[4];
   float emission[4];
   uint32_t flags;  // kRender* bits
@@ -38,7 +38,6 @@ cudaError_t light_pass(const uint32_t* old_grid, const uint32_t* new_grid, const
 // The fragment reads levels above 0 only through their alpha (the occlusion's
 // textureLod(...).a), so those levels are kept as alpha alone: the same box-filter sums of
 // the alpha channel, a quarter of the bytes.
-constexpr int kMaxMipLevels = 24;
 // The occlusion's textureLod calls use the integer lods 0 .. 6.
 constexpr int kOccLods = 7;
 // What the composite samples: the colour field (level 0) and, for lod l = 1 .. 6, the alpha
@@ -55,29 +54,54 @@ struct CompositeSrc {
 constexpr float kBlurSideWeight[3] = {0.606530666f, 0.704688072f, 0.818730772f};
 // Size of the next level: halved, at least 1.
 inline int mip_next(int n) { return n > 1 ? n / 2 : 1; }
-// output_color as render_color, plus (alpha1 != null) the pyramid's level-1 alpha,
-// mip_next(W) x mip_next(H): a cell's alpha is its material's colour alpha, so the level
-// comes from the same pass instead of a second read of the RGBA field.
-cudaError_t render_color_mip(const uint32_t* grid, const float* noise, float4* out, float* alpha1, int W, int H,
+// The pyramid levels the composite reads (alpha only): levels 1 .. levels - 1, at most 6.
+struct MipLevels {
+  float* level[kOccLods];  // [0] is unused
+  int w[kOccLods], h[kOccLods];
+  int levels;
+};
+// output_color as render_color, plus the pyramid's alpha levels (mip.levels <= 1: none): a
+// cell's alpha is its material's colour alpha, so they come from the same pass instead of a
+// second read of the RGBA field.
+cudaError_t render_color_mip(const uint32_t* grid, const float* noise, float4* out, const MipLevels& mip, int W, int H,
                              const RenderMat* mats, int nmat, cudaStream_t s);
-// The next alpha level (mip_next(sw) x mip_next(sh)) from an alpha level.
-cudaError_t render_mip_alpha(const float* src, int sw, int sh, float* dst, cudaStream_t s);
+// A coordinate's two bilinear taps along one axis of a texture: the wrapped indices, and the
+// weights of the second and of the first.
+struct alignas(16) Taps {
+  int i0, i1;
+  float a, ia;
+};
 // Column and row tables of the composite, functions of the field's size only (built once):
-// u = (c + 0.5) / W and the column of its nearest texel, the pixelated u of each column
-// pair (floor(u / d) * d at its even column, d = 1 / (W / 2)), and per row v, its nearest
-// row and the pixelated v.  Arrays hold round_up(W + 1, 4) / round_up(H + 1, 4) entries, so
-// that the pair loads of an odd last column or row stay in bounds.
+// u = (c + 0.5) / W and the column of its nearest texel; per column pair the nearest column and
+// the taps of its pixelated u (floor(u / d) * d at its even column, d = 1 / (W / 2)); per row v,
+// its nearest row, the pixelated v and that one's nearest row and taps.  Taps [l * lw + pair] /
+// [l * lh + row]: l = 0 along the light field, l >= 1 along the alpha level in slot l.  Column and
+// row arrays hold round_up(n + 1, 4) entries, so that the pair loads of an odd last column or
+// row stay in bounds.
 struct CompositeCoords {
   const float* u;
-  const int* ix;
-  const float* pu;
+  const int *ix, *ncol;
   const float* v;
   const int* iy;
   const float* pv;
+  const int* nrow;
+  const Taps *col, *row;
+  int lw, lh;
+};
+struct CompositeTable {  // the same, to be filled
+  float* u;
+  int *ix, *ncol;
+  float* v;
+  int* iy;
+  float* pv;
+  int* nrow;
+  Taps *col, *row;
+  int lw, lh;
 };
 size_t composite_coords_bytes(int W, int H);
-// Fills `buf` (composite_coords_bytes(W, H), 16-byte aligned) and points `out` into it.
-cudaError_t render_composite_coords(void* buf, int W, int H, CompositeCoords* out, cudaStream_t s);
+// Fills `buf` (composite_coords_bytes(W, H), 16-byte aligned) for src's sizes and points `out`
+// into it.
+cudaError_t render_composite_coords(void* buf, const CompositeSrc& src, CompositeCoords* out, cudaStream_t s);
 cudaError_t render_composite(const CompositeSrc& src, const CompositeCoords& coords, const float4* light,
                              const float4* bg, int bw, int bh, const float w_side[3], float4* out, cudaStream_t s);
 

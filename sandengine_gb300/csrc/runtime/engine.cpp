@@ -458,7 +458,7 @@ Status World::light_frame() {
   return Status::Ok();
 }
 
-Status World::render_color(float* alpha1) {
+Status World::render_color(const MipLevels* mip) {
   TraceRange trace("se_world_render_color");
   if (halo >= 0) return {SE_ERR_INVALID_ARGUMENT, "colours are rendered for whole worlds"};
   if (!d_noise) {
@@ -475,8 +475,8 @@ Status World::render_color(float* alpha1) {
     Status s = timing_begin(2, (long long)W * H, 1, &t);
     if (!s.ok()) return s;
   }
-  if (alpha1)
-    SE_CUDA(render_color_mip(buf[cur], d_noise, d_color, alpha1, W, H, rs->d_render, rs->num_materials(), stream));
+  if (mip)
+    SE_CUDA(render_color_mip(buf[cur], d_noise, d_color, *mip, W, H, rs->d_render, rs->num_materials(), stream));
   else
     SE_CUDA(se::rt::render_color(buf[cur], d_noise, d_color, W, H, rs->d_render, rs->num_materials(), stream));
   if (t) SE_CUDA(cudaEventRecord(t->b, stream));
@@ -486,25 +486,26 @@ Status World::render_color(float* alpha1) {
 Status World::composite(const float* bg, int bw, int bh) {
   TraceRange trace("se_world_composite");
   if (bg && (bw <= 0 || bh <= 0)) return {SE_ERR_INVALID_ARGUMENT, "background size must be positive"};
-  // pyramid sizes (level 0 is the colour field); the alpha levels are allocated once, and a
-  // 1 x 1 field keeps a copy of its alpha in place of level 1
-  int lw[kMaxMipLevels], lh[kMaxMipLevels], n = 1;
-  lw[0] = W;
-  lh[0] = H;
-  for (; (lw[n - 1] > 1 || lh[n - 1] > 1) && n < kMaxMipLevels; ++n) {
-    lw[n] = mip_next(lw[n - 1]);
-    lh[n] = mip_next(lh[n - 1]);
+  // pyramid levels 1 .. 6 (level 0 is the colour field, no larger lod is sampled); the alpha
+  // levels are allocated once, and a 1 x 1 field keeps a copy of its alpha in place of level 1
+  MipLevels mip{};
+  int n = 1;
+  mip.w[0] = W;
+  mip.h[0] = H;
+  for (; (mip.w[n - 1] > 1 || mip.h[n - 1] > 1) && n < kOccLods; ++n) {
+    mip.w[n] = mip_next(mip.w[n - 1]);
+    mip.h[n] = mip_next(mip.h[n - 1]);
   }
+  mip.levels = n;
   for (int l = (int)mips.size() + 1; l < std::max(n, 2); ++l) {
     float* m = nullptr;
-    cudaError_t e = cudaMalloc(&m, (l < n ? (size_t)lw[l] * (size_t)lh[l] : 1) * sizeof(float));
+    cudaError_t e = cudaMalloc(&m, (l < n ? (size_t)mip.w[l] * (size_t)mip.h[l] : 1) * sizeof(float));
     if (e != cudaSuccess) return {SE_ERR_OUT_OF_MEMORY, std::string("cudaMalloc: ") + cudaGetErrorString(e)};
     mips.push_back(m);
   }
-  // colours and level 1 in one pass, then the smaller levels
-  Status s = render_color(n > 1 ? mips[0] : nullptr);
+  for (int l = 1; l < n; ++l) mip.level[l] = mips[(size_t)l - 1];
+  Status s = render_color(&mip);  // colours and the pyramid in one pass
   if (!s.ok()) return s;
-  for (int l = 2; l < n; ++l) SE_CUDA(render_mip_alpha(mips[(size_t)l - 2], lw[l - 1], lh[l - 1], mips[(size_t)l - 1], stream));
   if (n == 1)
     SE_CUDA(cudaMemcpyAsync(mips[0], &d_color->w, sizeof(float), cudaMemcpyDeviceToDevice, stream));
   CompositeSrc src{};
@@ -514,8 +515,8 @@ Status World::composite(const float* bg, int bw, int bh) {
   for (int l = 1; l < kOccLods; ++l) {
     const int lv = std::max(1, std::min(l, n - 1));  // the level textureLod reads at lod l
     src.alpha[l] = mips[(size_t)lv - 1];
-    src.aw[l] = lv < n ? lw[lv] : 1;
-    src.ah[l] = lv < n ? lh[lv] : 1;
+    src.aw[l] = lv < n ? mip.w[lv] : 1;
+    src.ah[l] = lv < n ? mip.h[lv] : 1;
   }
   const float4* bgd = nullptr;
   if (bg) {
@@ -538,7 +539,7 @@ Status World::composite(const float* bg, int bw, int bh) {
   if (!d_coords) {
     cudaError_t e = cudaMalloc(&d_coords, composite_coords_bytes(W, H));
     if (e != cudaSuccess) return {SE_ERR_OUT_OF_MEMORY, std::string("cudaMalloc: ") + cudaGetErrorString(e)};
-    SE_CUDA(render_composite_coords(d_coords, W, H, &coords, stream));
+    SE_CUDA(render_composite_coords(d_coords, src, &coords, stream));
   }
   Timed* t = nullptr;
   if (timing) {

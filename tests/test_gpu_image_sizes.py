@@ -1,0 +1,34 @@
+"""Light, colours, alpha pyramid and composite at sizes around the passes' dispatch lines and tile
+edges: the light pass takes tiles of 4 rows up to 2^20 cells and of 16 rows beyond (several
+launches past 65535 row blocks), the colour pass reduces pyramid levels 1-4 from 16 x 8 cells a warp
+and 64 x 16 a CTA, and a second kernel levels 5 and 6.  Bit-exact against the oracle port."""
+import numpy as np
+import pytest
+
+from sandengine_gb300 import workloads as wl
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("shape", [(1024, 1024), (1025, 1024), (65, 17), (63, 15), (16, 8), (32, 33), (64, 1), (1, 64),
+                                   (31, 127), (129, 66), (3, 262150)])
+def test_light_and_composite_match_port(se, rulesets, ports, shape):
+    W, H = shape
+    P = ports["twelve_materials"]
+    sim = se.Simulation(se.parse_string(rulesets["twelve_materials"]), (W, H))
+    g = wl.patch_fill(W, H, 6, *wl.twelve_fill_spec(), patch=8)
+    sim.grid = g
+    sim.params.frame = 3
+    sim.set_light(True)
+    sim.run_frames(3)
+    light = np.zeros((H, W, 4), dtype=np.float32)
+    for f in (4, 5, 6):
+        old = g.copy()
+        P.step(g, f)
+        light = P.light(old, g, light)
+    assert np.array_equal(sim.grid, g)
+    assert np.array_equal(sim.output_light.view(np.uint32), light.view(np.uint32))
+    col = P.color(g)
+    got = sim.composite()
+    assert np.array_equal(got.view(np.uint32), P.composite(col, light).view(np.uint32))
+    assert np.array_equal(sim.output_color.view(np.uint32), col.view(np.uint32))
