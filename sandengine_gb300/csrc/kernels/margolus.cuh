@@ -677,6 +677,24 @@ __device__ __forceinline__ void se_tile_edits(uint8_t* sm, int SW, int SH, int g
   }
 }
 
+// The four cells (gx .. gx + 3, gy) of the grid whose rows [ya, yb) src holds; WALL outside it.
+// vec: rows are multiples of four cells and gx is a multiple of 4.
+__device__ __forceinline__ uint4 se_load_quad(const uint32_t* __restrict__ src, int W, int gx, int gy, int ya, int yb,
+                                              bool vec) {
+  uint4 v = make_uint4(SE_WALL, SE_WALL, SE_WALL, SE_WALL);
+  if (gy < ya || gy >= yb) return v;
+  const uint32_t* p = src + (size_t)(gy - ya) * W + gx;
+  if (vec) {
+    if (gx >= 0 && gx < W) v = __ldg(reinterpret_cast<const uint4*>(p));
+  } else {
+    if (gx >= 0 && gx < W) v.x = __ldg(p);
+    if (gx + 1 >= 0 && gx + 1 < W) v.y = __ldg(p + 1);
+    if (gx + 2 >= 0 && gx + 2 < W) v.z = __ldg(p + 2);
+    if (gx + 3 >= 0 && gx + 3 < W) v.w = __ldg(p + 3);
+  }
+  return v;
+}
+
 // Rule sets with a block transition table of 4-bit keys run their multi-frame tiles with two
 // cells per byte (nibble.cuh), unless their rules compare hash values besides the mirror test and use
 // all 16 ids (SE_NIB needs id 15 to mark blocks).
@@ -712,7 +730,7 @@ __device__ __forceinline__ void se_tile_edits(uint8_t* sm, int SW, int SH, int g
 // through the read-only cache.
 #define SE_NIB_SHARED (SE_NMAT <= 8)
 #define SE_NIB_ENTRIES (SE_NIB_SHARED ? SE_NMAT * SE_NMAT * SE_NMAT * SE_NMAT : 65536)
-#define SE_NIB_BOUNDS ((SE_NIB_ENTRIES + 2) & ~1)  // the bound table's first word
+#define SE_NIB_BOUNDS ((SE_NIB_ENTRIES + 4) & ~3)  // the bound table's first word
 // Launch bounds of the multi-frame tile kernels: up to 64 registers, for eight lookups and eight hashes of
 // a lane in flight (32 warps an SM; 40 or 48 at 48 or 40 registers ran 1% and 5% slower).
 #define SE_TILE_BOUNDS(NT) __launch_bounds__(NT, 1024 / NT)
@@ -796,24 +814,23 @@ __device__ __forceinline__ void se_tile_run(const uint32_t* __restrict__ src, ui
       }
     }
   } else {
-    for (int i = threadIdx.x; i < WPR * SH; i += NT) {
-      const int r = i / WPR, c = i - r * WPR;
-      const int gy = gy0 + r, gx = gx0 + 4 * c;
-      uint32_t packed;
-      if (gy < ya || gy >= yb) {
-        packed = 0x02020202u;
-      } else if (vec && gx >= 0 && gx + 3 < W) {
-        const uint4 v = __ldg(reinterpret_cast<const uint4*>(src + (size_t)(gy - ya) * W + gx));
-        packed = se_norm(v.x) | (se_norm(v.y) << 8) | (se_norm(v.z) << 16) | (se_norm(v.w) << 24);
-      } else {
-        packed = 0;
-        for (int e = 0; e < 4; ++e) {
-          const int x = gx + e;
-          const uint32_t id = (x >= 0 && x < W) ? se_norm(__ldg(src + (size_t)(gy - ya) * W + x)) : SE_WALL;
-          packed |= id << (8 * e);
-        }
+    // As above, four groups of four cells in flight per thread (one at a time, a small world's
+    // launch is mostly the latency of nine loads one after the other).
+    constexpr int NL = WPR * SH;
+    for (int i0 = threadIdx.x; i0 < NL; i0 += 4 * NT) {
+      uint4 v[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const int i = i0 + u * NT, r = i / WPR, c = i - r * WPR;
+        v[u] = se_load_quad(src, W, i < NL ? gx0 + 4 * c : W, gy0 + r, ya, yb, vec);
       }
-      *reinterpret_cast<uint32_t*>(sm + r * SW + 4 * c) = packed;
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const int i = i0 + u * NT;
+        if (i < NL)
+          reinterpret_cast<uint32_t*>(sm)[i] = se_norm(v[u].x) | (se_norm(v[u].y) << 8) | (se_norm(v[u].z) << 16) |
+                                               (se_norm(v[u].w) << 24);
+      }
     }
   }
   __syncthreads();

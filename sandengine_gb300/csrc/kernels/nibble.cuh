@@ -139,6 +139,23 @@ __device__ __forceinline__ uint32_t se_signs(uint32_t a, uint32_t b) {
 #endif
 }
 
+// Copies a shared reduced table into shared memory, 16 bytes a thread and step, asynchronously
+// (both ends hold whole groups of four words); se_nib_table_ready before the barrier.
+__device__ __forceinline__ void se_nib_copy_table(uint32_t* tab, const uint32_t* __restrict__ gtab, int nt) {
+#if SE_NIB_SHARED && defined(__CUDA_ARCH__)
+  for (int i = threadIdx.x; i < (SE_NIB_ENTRIES + 3) / 4; i += nt)
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 16;" ::"r"(
+                     (unsigned)__cvta_generic_to_shared(tab + 4 * i)),
+                 "l"(gtab + 4 * i)
+                 : "memory");
+#endif
+}
+__device__ __forceinline__ void se_nib_table_ready() {
+#if SE_NIB_SHARED && defined(__CUDA_ARCH__)
+  asm volatile("cp.async.wait_all;" ::: "memory");
+#endif
+}
+
 // The reduced table's entries of the four blocks of row words T and B.
 template <int NT>
 __device__ __forceinline__ void se_nib_lookup(uint32_t T, uint32_t B, uint32_t e[4], const uint32_t* tab,
@@ -412,10 +429,7 @@ __device__ __forceinline__ void se_nib_run(const uint32_t* __restrict__ src, uin
   const uint32_t* gtab = reinterpret_cast<const uint32_t*>(reinterpret_cast<const uint8_t*>(lut) + SE_NIB_OFF);
   uint32_t* tab = sm + G::TABLE;
   const uint32_t umask = NT == 1 ? se_nib_static_mask(lut) : __ldg(gtab + SE_NIB_ENTRIES);
-#if SE_NIB_SHARED
-  if (NT != 1)
-    for (int i = threadIdx.x; i < SE_NIB_ENTRIES; i += NT) tab[i] = __ldg(gtab + i);
-#endif
+  se_nib_copy_table(tab, gtab, NT);
   const int gx0 = X0 - G::HX, gy0 = Y0 - G::HY;
   const bool vec = (W & 3) == 0;
   constexpr int HPR = G::SW / 4;  // half-words (four cells) per row
@@ -452,27 +466,23 @@ __device__ __forceinline__ void se_nib_run(const uint32_t* __restrict__ src, uin
       }
     }
   } else {
-    for (int i = threadIdx.x; i < HPR * G::SH; i += NT) {
-      const int r = i / HPR, c = i - r * HPR;
-      const int gy = gy0 + r, gx = gx0 + 4 * c;
-      uint32_t packed = 0x2222u;
-      if (gy >= ya && gy < yb && gx + 3 >= 0 && gx < W) {
-        const uint32_t* p = src + (size_t)(gy - ya) * W;
-        if (vec && gx >= 0 && gx + 3 < W) {
-          packed = se_nib_pack(__ldg(reinterpret_cast<const uint4*>(p + gx)));
-        } else {
-          uint32_t id[4];
+    // As above, with a check of each group of four cells.
+    constexpr int NL = HPR * G::SH;
+    for (int i0 = threadIdx.x; i0 < NL; i0 += 4 * NT) {
+      uint4 v[4];
 #pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            const int x = gx + e;
-            id[e] = (x >= 0 && x < W) ? __ldg(p + x) : SE_WALL;
-          }
-          packed = se_nib_pack(make_uint4(id[0], id[1], id[2], id[3]));
-        }
+      for (int u = 0; u < 4; ++u) {
+        const int i = i0 + u * NT, r = i / HPR, c = i - r * HPR;
+        v[u] = se_load_quad(src, W, i < NL ? gx0 + 4 * c : W, gy0 + r, ya, yb, vec);
       }
-      sh[r * (2 * G::STRIDE) + c] = (uint16_t)packed;
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const int i = i0 + u * NT, r = i / HPR, c = i - r * HPR;
+        if (i < NL) sh[r * (2 * G::STRIDE) + c] = (uint16_t)se_nib_pack(v[u]);
+      }
     }
   }
+  se_nib_table_ready();
   __syncthreads();
 
   const bool edge = gx0 < 0 || gy0 < 0 || gx0 + G::SW > W || gy0 + G::SH > H;
@@ -547,13 +557,12 @@ __device__ __forceinline__ void se_nib_resident(const SeWorldDesc& w, int frames
   uint32_t* tab = sm + ((stride * rows + 3) & ~3);
 #if defined(__CUDA_ARCH__)
   const uint32_t umask = __ldg(gtab + SE_NIB_ENTRIES);
-#if SE_NIB_SHARED
-  for (int i = threadIdx.x; i < SE_NIB_ENTRIES; i += nt) tab[i] = __ldg(gtab + i);
-#endif
+  se_nib_copy_table(tab, gtab, nt);
 #else
   const uint32_t umask = se_nib_static_mask(lut);
 #endif
   for (int i = threadIdx.x; i < stride * rows; i += nt) sm[i] = 0x22222222u;
+  se_nib_table_ready();
   __syncthreads();
   const uint32_t* src = w.cur ? w.buf1 : w.buf0;
   uint32_t* dst = (w.cur ^ out_flip) ? w.buf1 : w.buf0;

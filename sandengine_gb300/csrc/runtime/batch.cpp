@@ -25,7 +25,7 @@ Status cuda_fail(const char* what, cudaError_t e) {
 size_t resident_bytes(int W, int H, const LutShape& lut) {
   if (lut.nib_entries) {
     const size_t stride = 2 * (((size_t)W + 5 + 15) / 16) + 2, rows = (size_t)H + 2;
-    return (((stride * rows + 3) & ~(size_t)3) + (lut.nib_shared ? lut.nib_entries : 0)) * 4;
+    return (((stride * rows + 3) & ~(size_t)3) + (lut.nib_shared ? (lut.nib_entries + 3) & ~3ull : 0)) * 4;
   }
   const size_t SW = (size_t)(((W + 7) & ~7) + 8), SH = (size_t)H + 2;
   const size_t cap = (SW / 8) * (SH / 2);
@@ -265,7 +265,7 @@ Status Batch::autotune(int reps, int* best_k) {
     for (int w : tiled) tiled_cells += (long long)desc[(size_t)w].W * desc[(size_t)w].H;
     double best_rate = 0;
     for (const TileVariant& v : tile_variants()) {
-      if (!v.fits(rs->lut_shape())) continue;
+      if (!v.tuned(rs->lut_shape(), tiled_cells)) continue;
       Status s = set_variant(&v);
       if (!s.ok()) return s;
       const size_t smem = tile_smem_bytes(v, rs->lut_shape());

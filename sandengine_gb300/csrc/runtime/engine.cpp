@@ -190,7 +190,7 @@ Status World::autotune(int reps, int* best_k) {
   double best_multi = 0, best_one = 0;
   const TileVariant *vm = nullptr, *v1 = nullptr;
   for (const TileVariant& v : tile_variants()) {
-    if (!v.fits(rs->lut_shape())) continue;
+    if (!v.tuned(rs->lut_shape(), (long long)W * H)) continue;
     Status s = launch_tiles(f0, v.kmax, &v, false);  // warm-up
     if (!s.ok()) return s;
     SE_CUDA(cudaEventRecord(a, stream));

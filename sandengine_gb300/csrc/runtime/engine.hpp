@@ -53,7 +53,7 @@ struct Ruleset {
     if (s.entries && s.static_words == keys / 32 && (n <= 15 || !prob)) {  // SE_NIB in the kernels
       s.nib_shared = n <= 8;
       s.nib_entries = s.nib_shared ? n * n * n * n : keys;
-      s.nib_words = ((s.nib_entries + 2) & ~1ull) + (prob ? 2 * keys : 0);  // SE_NIB_BOUNDS
+      s.nib_words = ((s.nib_entries + 4) & ~3ull) + (prob ? 2 * keys : 0);  // SE_NIB_BOUNDS
     }
     return s;
   }

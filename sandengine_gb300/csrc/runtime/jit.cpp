@@ -30,14 +30,26 @@ std::string TileVariant::edit_name() const {
 // (16-bit offsets in the chunk list).  The arrays of 4-bit tiles take whole warp items of
 // 32 x 32 cells, tile and halo together, so their shapes are 32 n - 2 halo.
 const std::vector<TileVariant>& tile_variants() {
-  constexpr int B = TileVariant::kByte, N = TileVariant::kNibble;
+  constexpr int B = TileVariant::kByte | TileVariant::kTuned, N = TileVariant::kNibble,
+                NT = TileVariant::kNibble | TileVariant::kTuned;
   static const std::vector<TileVariant> v = {
-      {128, 64, 1, 256, B | N}, {256, 32, 1, 256, B | N}, {128, 32, 1, 256, B | N}, {128, 64, 2, 256, B},
-      {128, 64, 4, 256, B},     {128, 64, 8, 256, B},     {128, 128, 8, 256, B},    {128, 128, 16, 256, B},
-      {256, 64, 4, 256, B},     {64, 64, 4, 256, B},      {256, 128, 8, 512, B},    {192, 128, 8, 256, B},
-      {256, 128, 4, 512, B},    {256, 64, 8, 256, B},
-      {120, 120, 4, 128, N},    {56, 56, 4, 128, N},      {112, 112, 8, 128, N},    {112, 48, 8, 128, N},
-      {48, 48, 8, 128, N},      {240, 176, 8, 256, N},    {240, 240, 8, 256, N},    {96, 96, 16, 128, N},
+      {128, 64, 1, 256, B | N},  {256, 32, 1, 256, B | N}, {128, 32, 1, 256, B | N}, {128, 64, 2, 256, B},
+      {128, 64, 4, 256, B},      {128, 64, 8, 256, B},     {128, 128, 8, 256, B},    {128, 128, 16, 256, B},
+      {256, 64, 4, 256, B},      {64, 64, 4, 256, B},      {256, 128, 8, 512, B},    {192, 128, 8, 256, B},
+      {256, 128, 4, 512, B},     {256, 64, 8, 256, B},
+      // 32x32 and 48x48 for the latency of small worlds, the large ones for the rate of large ones,
+      // 96x96 between (us a frame, four materials, 32x32_k16 / 48x48_k8 / 96x96_k16 / 112x112_k8 /
+      // 240x176_k8: 256^2 0.66 / 1.07 / 1.18 / 1.60 / 3.64, 1024^2 1.31 / 1.34 / 1.18 / 1.61 / 3.41, 4096^2 14.4
+      // / 8.7 / 7.2 / 7.0 / 6.5; three 4096^2 worlds at once, 60 frames of one: 852 / 489 / 387 / 362 / 313 us).
+      // The autotuner tries those whose range holds the world; 120x120 serves callers that ask for
+      // 2 to 4 frames a launch.
+      {120, 120, 4, 128, N},
+      {112, 112, 8, 256, NT, 1 << 18},
+      {48, 48, 8, 128, NT, 0, 1 << 23},
+      {240, 176, 8, 256, NT, 1 << 22},
+      {240, 240, 8, 256, NT, 1 << 23},
+      {96, 96, 16, 256, NT, 0, 1 << 22},
+      {32, 32, 16, 128, NT, 0, 1 << 20},
   };
   return v;
 }
@@ -188,7 +200,7 @@ size_t tile_smem_bytes(const TileVariant& t, const LutShape& lut) {
     const size_t sw16 = (size_t)(t.sw() + 15) / 16, wpr = 2 * ((sw16 + 1) / 2 * 2);
     const size_t stride = wpr + (wpr % 4 == 0 ? 2 : 4);
     const size_t rows = 32 * (((size_t)(t.sh() + 1) / 2 + 15) / 16) + 1;
-    return (((stride * rows + 3) & ~(size_t)3) + (lut.nib_shared ? lut.nib_entries : 0)) * 4;
+    return (((stride * rows + 3) & ~(size_t)3) + (lut.nib_shared ? (lut.nib_entries + 3) & ~3ull : 0)) * 4;
   }
   size_t b = (t.smem_bytes() + 15) & ~(size_t)15;
   // 48-byte header (slack, list counters, uniform-material flags), then the per-step list

@@ -24,9 +24,14 @@ struct LutShape {
 // A tile-kernel instantiation: TW x TH output cells, up to KMAX frames per launch.
 struct TileVariant {
   int tw, th, kmax, nt;
-  enum { kByte = 1, kNibble = 2 };
-  int use;  // the kinds of tile it is chosen for (set_tile may ask for any)
+  enum { kByte = 1, kNibble = 2, kTuned = 4 };
+  int use;  // the kinds of tile it is chosen for, and whether by the autotuner (set_tile may ask for any)
+  long long min_cells = 0, max_cells = 1ll << 62;
   bool fits(const LutShape& lut) const { return use & (lut.nib_entries ? kNibble : kByte); }
+  // Whether the autotuner tries it on `cells` cells (of one world, or of a batch's tiled worlds).
+  bool tuned(const LutShape& lut, long long cells) const {
+    return fits(lut) && (use & kTuned) && cells >= min_cells && cells <= max_cells;
+  }
   std::string name() const;        // single-world kernel
   std::string edit_name() const;   // single-world kernel with the first frame's edit pass
   std::string multi_name() const;  // many-world (tile job list) kernel
