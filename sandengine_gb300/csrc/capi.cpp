@@ -385,7 +385,7 @@ SE_API int se_world_get_tile(const se_world* w, int* tile_w, int* tile_h, int* k
     if (!w || !tile_w || !tile_h || !k) return fail(SE_ERR_INVALID_ARGUMENT, "null argument");
     const auto& W = *w->w;
     const se::rt::TileVariant* v = W.steps_per_launch > 0 ? nullptr : W.fused;
-    if (!v) v = se::rt::pick_variant(std::max(1, W.steps_per_launch), W.rs->lut_shape());
+    if (!v) v = se::rt::pick_variant(std::max(1, W.steps_per_launch), W.rs->lut_shape(), (long long)W.W * W.H);
     *tile_w = v ? v->tw : 0;
     *tile_h = v ? v->th : 0;
     *k = v ? v->kmax : 0;
@@ -632,7 +632,7 @@ SE_API int se_batch_autotune(se_batch* b, int reps, int* best_k) {
 SE_API int se_batch_set_steps_per_launch(se_batch* b, int k) {
   return guard([&] {
     if (!b || k < 1) return fail(SE_ERR_INVALID_ARGUMENT, "k must be >= 1");
-    const se::rt::TileVariant* v = se::rt::pick_variant(k, b->b->rs->lut_shape());
+    const se::rt::TileVariant* v = se::rt::pick_variant(k, b->b->rs->lut_shape(), -1);
     if (!v) return fail(SE_ERR_INVALID_ARGUMENT, "no kernel variant for this many frames per launch");
     b->b->steps_per_launch = k;
     return ret(b->b->set_variant(v));

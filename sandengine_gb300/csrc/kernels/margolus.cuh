@@ -755,9 +755,9 @@ __device__ __forceinline__ void se_tile_run(const uint32_t* __restrict__ src, ui
                                             int ya, int yb, const SeEditParams* __restrict__ edits = nullptr,
                                             int nedits = 0) {
 #ifdef SE_NIB
-  // One-frame launches keep byte tiles: they run at the memory's speed, and packing the cells
+  // Large one-frame tiles keep bytes: they run at the memory's speed, and packing the cells
   // costs more than it saves there (85 against 108 us a frame of an 8192 x 8192 world).
-  if constexpr (KMAX > 1) {
+  if constexpr (KMAX > 1 || TW * TH <= 2048) {
     se_nib_run<TW, TH, KMAX, NT>(src, dst, W, H, f0, k, lut, X0, Y0, ya, yb, edits, nedits);
     return;
   }

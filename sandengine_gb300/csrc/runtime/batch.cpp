@@ -323,7 +323,7 @@ Status Batch::step(int F) {
     Status s = steps_per_launch > 0 ? Status::Ok() : autotune(2, nullptr);
     if (!s.ok()) return s;
     if (!variant) {
-      s = set_variant(pick_variant(steps_per_launch, rs->lut_shape()));
+      s = set_variant(pick_variant(steps_per_launch, rs->lut_shape(), -1));
       if (!s.ok()) return s;
     }
   }
@@ -353,7 +353,6 @@ Status Batch::step(int F) {
 
 Status Batch::step_plain(int F) {
   if (F < 0) return {SE_ERR_INVALID_ARGUMENT, "nframes must be >= 0"};
-  const TileVariant* v1 = pick_variant(1, rs->lut_shape());
   for (int f = 0; f < F; ++f) {
     for (auto& d : desc) {
       const int fr = d.frame + 1;
@@ -362,6 +361,7 @@ Status Batch::step_plain(int F) {
       } else {
         const uint32_t* src = d.cur ? d.buf1 : d.buf0;
         uint32_t* dst = d.cur ? d.buf0 : d.buf1;
+        const TileVariant* v1 = pick_variant(1, rs->lut_shape(), (long long)d.W * d.H);
         Status s = launch_tile_kernel(*rs, *v1, src, dst, d.W, d.H, fr, 1, 0, d.H, stream);
         if (!s.ok()) return s;
         d.cur ^= 1;

@@ -369,15 +369,15 @@ Status World::step(int nframes, const se_modification* mods, int nmods) {
   while (nlive < nseen && mods[nlive].mod_size != 0) ++nlive;  // falling_sand.glsl:139-141
   const TileVariant* vmulti = nullptr;
   if (steps_per_launch > 0) {
-    vmulti = pick_variant(steps_per_launch, rs->lut_shape());
+    vmulti = pick_variant(steps_per_launch, rs->lut_shape(), (long long)W * H);
   } else {
     if (!fused && nframes >= 2) {
       Status s = autotune(2, nullptr);
       if (!s.ok()) return s;
     }
-    vmulti = fused ? fused : pick_variant(1, rs->lut_shape());
+    vmulti = fused ? fused : pick_variant(1, rs->lut_shape(), (long long)W * H);
   }
-  const TileVariant* vone = single ? single : pick_variant(1, rs->lut_shape());
+  const TileVariant* vone = single ? single : pick_variant(1, rs->lut_shape(), (long long)W * H);
   const int kdef = steps_per_launch > 0 ? steps_per_launch : vmulti->kmax;
   if (light[0]) {  // one frame at a time, each followed by the light pass
     for (int i = 0; i < nframes; ++i) {

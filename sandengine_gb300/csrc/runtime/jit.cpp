@@ -33,6 +33,10 @@ const std::vector<TileVariant>& tile_variants() {
   constexpr int B = TileVariant::kByte | TileVariant::kTuned, N = TileVariant::kNibble,
                 NT = TileVariant::kNibble | TileVariant::kTuned;
   static const std::vector<TileVariant> v = {
+      // one frame of a small world is the latency of a few CTAs: 4-bit tiles of 64 x 32 cells with
+      // their halo (us a launch, four materials, 56x30 / 128x64 bytes: 64^2 to 512^2 4.2 / 8.2, 1024^2
+      // 6.2 / 8.3, 2048^2 8.3 / 11.4; twelve 4.1 / 7.6, 6.2 / 8.3, 10.3 / 12.3)
+      {56, 30, 1, 128, NT, 0, 1 << 22},
       {128, 64, 1, 256, B | N},  {256, 32, 1, 256, B | N}, {128, 32, 1, 256, B | N}, {128, 64, 2, 256, B},
       {128, 64, 4, 256, B},      {128, 64, 8, 256, B},     {128, 128, 8, 256, B},    {128, 128, 16, 256, B},
       {256, 64, 4, 256, B},      {64, 64, 4, 256, B},      {256, 128, 8, 512, B},    {192, 128, 8, 256, B},
@@ -54,10 +58,14 @@ const std::vector<TileVariant>& tile_variants() {
   return v;
 }
 
-const TileVariant* pick_variant(int k, const LutShape& lut) {
+const TileVariant* pick_variant(int k, const LutShape& lut, long long cells) {
   const TileVariant* best = nullptr;
-  for (const TileVariant& t : tile_variants())
-    if (t.kmax >= k && t.fits(lut) && (!best || t.kmax < best->kmax)) best = &t;
+  for (bool ranged : {true, false}) {
+    if (best) break;
+    for (const TileVariant& t : tile_variants())
+      if (t.kmax >= k && t.fits(lut) && (!ranged || cells < 0 || t.holds(cells)) && (!best || t.kmax < best->kmax))
+        best = &t;
+  }
   return best;
 }
 
@@ -66,7 +74,7 @@ std::string kernel_source(const std::string& generated_rules) {
   o << SE_PRELUDE_SRC << "\n" << generated_rules << "\n" << SE_MARGOLUS_SRC << "\n"
     << SE_NIBBLE_SRC << "\n";
   for (const TileVariant& t : tile_variants()) {
-    const std::string bounds = (t.kmax > 1 ? "SE_TILE_BOUNDS(" : "__launch_bounds__(") + std::to_string(t.nt) + ") ";
+    const std::string bounds = (t.kmax > 1 || t.small() ? "SE_TILE_BOUNDS(" : "__launch_bounds__(") + std::to_string(t.nt) + ") ";
     o << "extern \"C\" __global__ void " << bounds << t.name()
       << "(const uint32_t* __restrict__ src, uint32_t* __restrict__ dst, int W, int H, int f0, int k,"
          " const uint16_t* __restrict__ lut, int ya, int yb) {\n"
@@ -196,7 +204,7 @@ Module::~Module() {
 }
 
 size_t tile_smem_bytes(const TileVariant& t, const LutShape& lut) {
-  if (lut.nib_entries && t.kmax > 1) {  // SeNib's array (nibble.cuh) and, when small, its reduced table
+  if (lut.nib_entries && (t.kmax > 1 || t.small())) {  // SeNib's array (nibble.cuh) and, when small, its reduced table
     const size_t sw16 = (size_t)(t.sw() + 15) / 16, wpr = 2 * ((sw16 + 1) / 2 * 2);
     const size_t stride = wpr + (wpr % 4 == 0 ? 2 : 4);
     const size_t rows = 32 * (((size_t)(t.sh() + 1) / 2 + 15) / 16) + 1;

@@ -30,8 +30,10 @@ struct TileVariant {
   bool fits(const LutShape& lut) const { return use & (lut.nib_entries ? kNibble : kByte); }
   // Whether the autotuner tries it on `cells` cells (of one world, or of a batch's tiled worlds).
   bool tuned(const LutShape& lut, long long cells) const {
-    return fits(lut) && (use & kTuned) && cells >= min_cells && cells <= max_cells;
+    return fits(lut) && (use & kTuned) && holds(cells);
   }
+  bool holds(long long cells) const { return cells >= min_cells && cells <= max_cells; }
+  bool small() const { return tw * th <= 2048; }  // one-frame tiles on 4-bit cells (se_tile_run)
   std::string name() const;        // single-world kernel
   std::string edit_name() const;   // single-world kernel with the first frame's edit pass
   std::string multi_name() const;  // many-world (tile job list) kernel
@@ -43,9 +45,9 @@ struct TileVariant {
   size_t smem_bytes() const { return (size_t)sw() * (size_t)sh(); }
 };
 const std::vector<TileVariant>& tile_variants();
-// The variant for k frames per launch: of those chosen for the rule set's tiles the first with
-// the fewest frames >= k.
-const TileVariant* pick_variant(int k, const LutShape& lut);
+// The variant for k frames per launch: of those chosen for the rule set's tiles and for worlds of
+// `cells` cells (-1: any) the first with the fewest frames >= k.
+const TileVariant* pick_variant(int k, const LutShape& lut, long long cells);
 
 // Dynamic shared memory of a tile launch: the u8 tile, then the per-step list of chunks to
 // evaluate; or the 4-bit tile and a small reduced table.  The block transition table and its

@@ -74,7 +74,7 @@ Status Server::set_frames_per_iteration(int k) {
   // throughput, 770 G cell-updates/s, against 690-734 G with 256x128, 128x128 or 256x64
   // tiles): their smaller halo loss on the large tiles does not make up for the waste on
   // the small sessions and the coarser work units of an iteration.
-  const TileVariant* v = pick_variant(k, rs->lut_shape());
+  const TileVariant* v = pick_variant(k, rs->lut_shape(), -1);
   if (!v || k < 1) return {SE_ERR_INVALID_ARGUMENT, "no kernel variant for this many frames per iteration"};
   variant = v;
   return Status::Ok();
@@ -608,7 +608,6 @@ Status Server::serve_plain(std::unique_lock<std::mutex>& lk) {
     std::stable_sort(pend.begin(), pend.end(),
                      [&](int a, int b) { return requests[(size_t)a].arrival_ms < requests[(size_t)b].arrival_ms; });
   }
-  const TileVariant* v1 = pick_variant(1, rs->lut_shape());
   size_t next = 0;
   for (;;) {
     int ri = -1;
@@ -649,6 +648,7 @@ Status Server::serve_plain(std::unique_lock<std::mutex>& lk) {
       if (f == 1) {
         SE_CUDA(cudaMemsetAsync(ss.buf(ss.cur), 0, (size_t)ss.W * ss.H * 4, stream));
       } else {
+        const TileVariant* v1 = pick_variant(1, rs->lut_shape(), (long long)ss.W * ss.H);
         st = launch_tile_kernel(*rs, *v1, ss.buf(ss.cur), ss.buf(ss.cur ^ 1), ss.W, ss.H, f, 1, 0, ss.H, stream);
         if (!st.ok()) return st;
         ss.cur ^= 1;

@@ -9,7 +9,7 @@ import pytest
 pytestmark = pytest.mark.gpu
 
 # (tile width, tile height, frames) of the shapes; sizes are derived from them
-SHAPES = [(120, 120, 4), (112, 112, 8), (48, 48, 8), (240, 176, 8), (240, 240, 8), (96, 96, 16), (32, 32, 16)]
+SHAPES = [(56, 30, 1), (120, 120, 4), (112, 112, 8), (48, 48, 8), (240, 176, 8), (240, 240, 8), (96, 96, 16), (32, 32, 16)]
 # several lanes compared: probability on lane 1, a condition on lane 2
 LANES_RULE = """
   shake:
