@@ -32,3 +32,15 @@ def test_light_and_composite_match_port(se, rulesets, ports, shape):
     got = sim.composite()
     assert np.array_equal(got.view(np.uint32), P.composite(col, light).view(np.uint32))
     assert np.array_equal(sim.output_color.view(np.uint32), col.view(np.uint32))
+
+
+@pytest.mark.parametrize("shape", [(97, 70), (1, 100), (100, 1), (32, 32), (33, 31), (2000, 3), (1048576, 1),
+                                   (3, 1048575), (1048573, 2)])
+def test_colour_noise_matches_port(se, rulesets, ports, shape):
+    """Tiles of 32 x 32 cells and their remainders, up to the longest sides, whose sines have
+    arguments beyond the range of the integer path."""
+    W, H = shape
+    sim = se.Simulation(se.parse_string(rulesets["twelve_materials"]), (W, H))
+    g = np.full((H, W), 3, dtype=np.uint32)
+    sim.grid = g
+    assert np.array_equal(sim.output_color.view(np.uint32), ports["twelve_materials"].color(g).view(np.uint32))
