@@ -220,7 +220,7 @@ Status launch_tile_kernel(const Ruleset& rs, const TileVariant& v, const uint32_
   if (ya < 0 || yb > H || ya >= yb) return {SE_ERR_INVALID_ARGUMENT, "tile rows outside the world"};
   if (edits && (nedits < 1 || nedits > SE_MAX_MODIFICATIONS))
     return {SE_ERR_INVALID_ARGUMENT, "an edit launch takes 1..256 modifications"};
-  cudaKernel_t kern = rs.module->get(edits ? v.edit_name() : v.name());
+  cudaKernel_t kern = rs.module->tile(v, edits != nullptr);
   const uint16_t* lut = rs.d_lut;
   // se_tile_impl's order; the edit variant adds the edit list (by value) and its length
   void* args[] = {(void*)&src, (void*)&dst, &W, &H, &f0, &k, (void*)&lut, &ya, &yb, (void*)edits, &nedits};
@@ -301,8 +301,7 @@ Status World::timing_read(int pass, double* ms, long long* launches, long long* 
 
 long long fill_edit_params(const Ruleset& rs, int W, int row0, int rows, const se_modification* mods, int nlive,
                            EditParams* out) {
-  EditParams& p = *out;
-  memset(&p, 0, sizeof p);
+  EditParams& p = *out;  // written up to the entries that the launch reads
   long long total = 0;
   const int nmat = rs.num_materials();
   for (int i = 0; i < nlive; ++i) {
@@ -367,6 +366,7 @@ Status World::step(int nframes, const se_modification* mods, int nmods) {
   int nlive = 0;
   const int nseen = std::min(nmods, SE_MAX_MODIFICATIONS);  // simulation.rs:205
   while (nlive < nseen && mods[nlive].mod_size != 0) ++nlive;  // falling_sand.glsl:139-141
+  const TileVariant* vone = single ? single : pick_variant(1, rs->lut_shape(), (long long)W * H);
   const TileVariant* vmulti = nullptr;
   if (steps_per_launch > 0) {
     vmulti = pick_variant(steps_per_launch, rs->lut_shape(), (long long)W * H);
@@ -375,9 +375,9 @@ Status World::step(int nframes, const se_modification* mods, int nmods) {
       Status s = autotune(2, nullptr);
       if (!s.ok()) return s;
     }
-    vmulti = fused ? fused : pick_variant(1, rs->lut_shape(), (long long)W * H);
+    if (single) vone = single;  // the autotuner's
+    vmulti = fused ? fused : vone;
   }
-  const TileVariant* vone = single ? single : pick_variant(1, rs->lut_shape(), (long long)W * H);
   const int kdef = steps_per_launch > 0 ? steps_per_launch : vmulti->kmax;
   if (light[0]) {  // one frame at a time, each followed by the light pass
     for (int i = 0; i < nframes; ++i) {

@@ -246,6 +246,8 @@ bool Module::load(const std::string& cubin, const LutShape& lut, std::string* er
     kernels[n] = k;
   }
   for (auto& t : tile_variants()) {
+    tiles.push_back(kernels[t.name()]);
+    tiles.push_back(kernels[t.edit_name()]);
     for (const std::string& n : {t.name(), t.edit_name(), t.multi_name(), t.serve_name()}) {
       e = cudaFuncSetAttribute((const void*)kernels[n], cudaFuncAttributeMaxDynamicSharedMemorySize,
                                (int)tile_smem_bytes(t, lut));

@@ -63,10 +63,15 @@ bool compile_cubin(const std::string& src, std::string* cubin, std::string* log)
 struct Module {
   cudaLibrary_t lib = nullptr;
   std::map<std::string, cudaKernel_t> kernels;
+  std::vector<cudaKernel_t> tiles;  // of each variant: the plain kernel, the one with edits
   size_t max_dyn_smem = 0;  // opt-in dynamic shared memory per CTA on this device
   ~Module();
   bool load(const std::string& cubin, const LutShape& lut, std::string* err);
   cudaKernel_t get(const std::string& name) const;
+  // The variant's kernel (t: an element of tile_variants()), without building its name.
+  cudaKernel_t tile(const TileVariant& t, bool edits) const {
+    return tiles[2 * (size_t)(&t - tile_variants().data()) + (edits ? 1 : 0)];
+  }
 };
 
 }  // namespace se::rt

@@ -15,6 +15,7 @@ from __future__ import annotations
 
 import ctypes
 import os
+import struct
 from dataclasses import dataclass, field
 from typing import List, Optional, Sequence, Tuple
 
@@ -37,11 +38,19 @@ class SimModification:
     mod_matID: int = 0
 
 
+_MOD = struct.Struct("=5i12x")  # SeModification
+assert _MOD.size == ctypes.sizeof(SeModification)
+
+
 def mods_to_c(mods: Sequence[SimModification]):
     arr = (SeModification * max(1, len(mods)))()
     for i, m in enumerate(mods):
-        arr[i].position[0], arr[i].position[1] = int(m.position[0]), int(m.position[1])
-        arr[i].mod_shape, arr[i].mod_size, arr[i].mod_matID = int(m.mod_shape), int(m.mod_size), int(m.mod_matID)
+        try:
+            p = m.position
+            _MOD.pack_into(arr, i * _MOD.size, p[0], p[1], m.mod_shape, m.mod_size, m.mod_matID)
+        except struct.error:  # not whole numbers of 32 bits: int() and ctypes truncate
+            arr[i].position[0], arr[i].position[1] = int(m.position[0]), int(m.position[1])
+            arr[i].mod_shape, arr[i].mod_size, arr[i].mod_matID = int(m.mod_shape), int(m.mod_size), int(m.mod_matID)
     return arr
 
 
