@@ -205,14 +205,14 @@ __device__ __forceinline__ float mip_texel(float a, float b, float c, float d, i
 // 4.1 + 11.4 -> 7.2, 4096 x 4096 66 + 39 -> 78, 8192 x 8192 250 + 54 -> 283.  64 x 64 cells a CTA with
 // all six levels reduced in shared memory kept too few loads in flight between its barriers
 // (8192 x 8192: 323 and 545 us with 256 and 1024 threads).
-__global__ void __launch_bounds__(256) se_color_mip_kernel(const uint32_t* __restrict__ grid,
-                                                           const float* __restrict__ noise, float4* __restrict__ out,
-                                                           const MipLevels mip, int W, int H,
-                                                           const RenderMat* __restrict__ mats, int nmat, int by0) {
-  __shared__ float s3[2][8];
-  const int lane = threadIdx.x & 31, wx = (threadIdx.x >> 5) & 3, wy = threadIdx.x >> 7;
-  const int by = by0 + blockIdx.y;
-  const int x = blockIdx.x * 32 + wx * 8 + (lane & 7), y = by * 8 + wy * 4 + (lane >> 3);
+// Block (bx, by) of 64 x 16 cells by threads t = 0 .. 255 (whole CTAs take part; blocks beyond the world
+// write nothing).
+__device__ __forceinline__ void color_mip_block(const uint32_t* __restrict__ grid, const float* __restrict__ noise,
+                                                float4* out, const MipLevels& mip, int W, int H,
+                                                const RenderMat* __restrict__ mats, int nmat, int bx, int by, int t,
+                                                float (*s3)[8]) {
+  const int lane = t & 31, wx = (t >> 5) & 3, wy = t >> 7;
+  const int x = bx * 32 + wx * 8 + (lane & 7), y = by * 8 + wy * 4 + (lane >> 3);
   const int c0 = 2 * x, r0 = 2 * y;
   float v = 0.0f;
   if (c0 < W && r0 < H) {
@@ -258,18 +258,36 @@ __global__ void __launch_bounds__(256) se_color_mip_kernel(const uint32_t* __res
   if (mip.levels <= 4) return;
   if (lane == 0 || lane == 4) s3[wy][wx * 2 + (lane >> 2)] = v;
   __syncthreads();
-  if (threadIdx.x < 4) {
-    const int i = threadIdx.x, tx = blockIdx.x * 4 + i;
+  if (t < 4) {
+    const int i = t, tx = bx * 4 + i;
     if (tx < mip.w[4] && by < mip.h[4])
       mip.level[4][(size_t)by * mip.w[4] + tx] =
           mip_texel(s3[0][2 * i], s3[0][2 * i + 1], s3[1][2 * i], s3[1][2 * i + 1], mip.w[3], mip.h[3]);
   }
 }
 
-// Levels 5 and 6 from level 4: a thread takes the 4 x 4 texels of level 4 under a texel of level 6.
-__global__ void __launch_bounds__(128) se_mip_tail_kernel(const MipLevels mip) {
+__global__ void __launch_bounds__(256) se_color_mip_kernel(const uint32_t* __restrict__ grid,
+                                                           const float* __restrict__ noise, float4* __restrict__ out,
+                                                           const MipLevels mip, int W, int H,
+                                                           const RenderMat* __restrict__ mats, int nmat, int by0) {
+  __shared__ float s3[2][8];
+  color_mip_block(grid, noise, out, mip, W, H, mats, nmat, blockIdx.x, by0 + blockIdx.y, threadIdx.x, s3);
+}
+
+// A load: of what an earlier launch wrote, or (SAME) this launch itself, before a barrier.
+template <bool SAME, class T>
+__device__ __forceinline__ T load(const T* p) {
+  if constexpr (SAME)
+    return *p;
+  else
+    return __ldg(p);
+}
+
+// Levels 5 and 6 from level 4: thread t takes the 4 x 4 texels of level 4 under a texel of level 6.
+template <bool SAME>
+__device__ __forceinline__ void mip_tail(const MipLevels& mip, int t) {
   const int w4 = mip.w[4], h4 = mip.h[4], w5 = mip.w[5], h5 = mip.h[5];
-  const int nx = (w5 + 1) / 2, t = blockIdx.x * 128 + threadIdx.x;
+  const int nx = (w5 + 1) / 2;
   const int X = t % nx, Y = t / nx;
   if (2 * Y >= h5) return;
   float a[4][4];
@@ -277,7 +295,7 @@ __global__ void __launch_bounds__(128) se_mip_tail_kernel(const MipLevels mip) {
   for (int j = 0; j < 4; ++j)
 #pragma unroll
     for (int i = 0; i < 4; ++i)
-      a[j][i] = __ldg(mip.level[4] + (size_t)min(4 * Y + j, h4 - 1) * w4 + min(4 * X + i, w4 - 1));
+      a[j][i] = load<SAME>(mip.level[4] + (size_t)min(4 * Y + j, h4 - 1) * w4 + min(4 * X + i, w4 - 1));
   float b[2][2];
 #pragma unroll
   for (int j = 0; j < 2; ++j)
@@ -288,6 +306,9 @@ __global__ void __launch_bounds__(128) se_mip_tail_kernel(const MipLevels mip) {
     }
   if (mip.levels > 6 && X < mip.w[6] && Y < mip.h[6])
     mip.level[6][(size_t)Y * mip.w[6] + X] = mip_texel(b[0][0], b[0][1], b[1][0], b[1][1], w5, h5);
+}
+__global__ void __launch_bounds__(128) se_mip_tail_kernel(const MipLevels mip) {
+  mip_tail<false>(mip, blockIdx.x * 128 + threadIdx.x);
 }
 
 // Light pass over a 64 x 4R tile per CTA.  The tile plus a one-cell ring is staged in
@@ -503,7 +524,7 @@ __device__ __forceinline__ Taps load_taps(const Taps* p) {
   return Taps{__float_as_int(v.x), __float_as_int(v.y), v.z, v.w};
 }
 // Column pair k and row r0.  IDX: the integer type that holds any texel's index.
-template <class IDX>
+template <class IDX, bool SAME>
 __device__ __forceinline__ Shared shared_terms(const CompositeSrc& m, const CompositeCoords& cc,
                                                const float4* __restrict__ light, int k, int r0, float ws0, float ws1,
                                                float ws2) {
@@ -522,15 +543,15 @@ __device__ __forceinline__ Shared shared_terms(const CompositeSrc& m, const Comp
   // seven distinct samples.  lod 0 is a magnification (level 0, nearest); lod l >= 1 reads
   // the alpha level in slot l, bilinearly.
   float s[kOccLods];
-  s[0] = __ldg(&m.color[(IDX)__ldg(cc.nrow + r0) * (IDX)m.w + (IDX)__ldg(cc.ncol + k)].w);
+  s[0] = load<SAME>(&m.color[(IDX)__ldg(cc.nrow + r0) * (IDX)m.w + (IDX)__ldg(cc.ncol + k)].w);
 #pragma unroll
   for (int l = 1; l < kOccLods; ++l) {
     const Taps c = load_taps(cc.col + (size_t)l * cc.lw + k), r = load_taps(cc.row + (size_t)l * cc.lh + r0);
     const Weights k = tap_weights(c, r);
     const IDX p = (IDX)r.i0 * (IDX)m.aw[l], q = (IDX)r.i1 * (IDX)m.aw[l];
     const float* A = m.alpha[l];
-    s[l] = lerp4(__ldg(A + (p + (IDX)c.i0)), __ldg(A + (p + (IDX)c.i1)), __ldg(A + (q + (IDX)c.i0)),
-                 __ldg(A + (q + (IDX)c.i1)), k.w00, k.w10, k.w01, k.w11);
+    s[l] = lerp4(load<SAME>(A + (p + (IDX)c.i0)), load<SAME>(A + (p + (IDX)c.i1)), load<SAME>(A + (q + (IDX)c.i0)),
+                 load<SAME>(A + (q + (IDX)c.i1)), k.w00, k.w10, k.w01, k.w11);
   }
   const float occ = fsub(1.0f, blurred_alpha(s[0], s[1], s[2], ws0));
   const float occ2 = fsub(1.0f, blurred_alpha(s[3], s[4], s[5], ws1));
@@ -577,14 +598,13 @@ __global__ void __launch_bounds__(256) se_composite_coords_kernel(CompositeTable
 // 14.1 M warp instructions instead of 17.8 M, 36.6 -> 27.1 us; 64 x 64 8.3 -> 4.3, 4096 x 4096
 // 181 -> 155 us = 5.2 TB/s of 48 B a pixel).  Tables rebuilt per CTA in shared memory cost what they
 // saved (35 and 189 us), as did one lane per pixel with the shared terms passed by shuffles.
-template <class IDX>
-__global__ void __launch_bounds__(256, 4) se_composite_kernel(const CompositeSrc m, const CompositeCoords cc,
-                                                              const float4* __restrict__ light,
-                                                              const float4* __restrict__ bg, int bw, int bh, float ws0,
-                                                              float ws1, float ws2, float4* __restrict__ out,
-                                                              int by0) {
+template <class IDX, bool SAME>
+__device__ __forceinline__ void composite_block(const CompositeSrc& m, const CompositeCoords& cc,
+                                                const float4* __restrict__ light, const float4* __restrict__ bg, int bw,
+                                                int bh, float ws0, float ws1, float ws2, float4* __restrict__ out,
+                                                int bx, int by, int t) {
   const int W = m.w, H = m.h;
-  const int k = blockIdx.x * 32 + (threadIdx.x & 31), c0 = 2 * k, r0 = 2 * ((by0 + blockIdx.y) * 8 + (threadIdx.x >> 5));
+  const int k = bx * 32 + (t & 31), c0 = 2 * k, r0 = 2 * (by * 8 + (t >> 5));
   if (c0 >= W || r0 >= H) return;
   // c0 and r0 are even: 8-byte aligned pair loads, in bounds up to index W / H
   const float2 us = __ldg(reinterpret_cast<const float2*>(cc.u + c0));
@@ -598,16 +618,16 @@ __global__ void __launch_bounds__(256, 4) se_composite_kernel(const CompositeSrc
 #pragma unroll
   for (int dr = 0; dr < 2; ++dr) {
     const IDX p = (IDX)(dr && down ? iys.y : iys.x) * (IDX)W;
-    cols[dr][0] = __ldg(m.color + (p + (IDX)ixs.x));
-    cols[dr][1] = __ldg(m.color + (p + (IDX)(two ? ixs.y : ixs.x)));
+    cols[dr][0] = load<SAME>(m.color + (p + (IDX)ixs.x));
+    cols[dr][1] = load<SAME>(m.color + (p + (IDX)(two ? ixs.y : ixs.x)));
   }
   const float ambient = 0.1f;
-  Shared S = shared_terms<IDX>(m, cc, light, k, r0, ws0, ws1, ws2);
+  Shared S = shared_terms<IDX, SAME>(m, cc, light, k, r0, ws0, ws1, ws2);
 #pragma unroll
   for (int dr = 0; dr < 2; ++dr) {
     if (dr == 1) {
       if (!down) break;
-      if (pvs.y != pvs.x) S = shared_terms<IDX>(m, cc, light, k, r0 + 1, ws0, ws1, ws2);
+      if (pvs.y != pvs.x) S = shared_terms<IDX, SAME>(m, cc, light, k, r0 + 1, ws0, ws1, ws2);
     }
     const float v = dr ? vs.y : vs.x;
     const float sky = fmul(0.5f, fsub(1.0f, dr ? pvs.y : pvs.x));
@@ -632,6 +652,46 @@ __global__ void __launch_bounds__(256, 4) se_composite_kernel(const CompositeSrc
       out[(size_t)(r0 + dr) * W + cx] = o;
     }
   }
+}
+
+template <class IDX>
+__global__ void __launch_bounds__(256, 4) se_composite_kernel(const CompositeSrc m, const CompositeCoords cc,
+                                                              const float4* __restrict__ light,
+                                                              const float4* __restrict__ bg, int bw, int bh, float ws0,
+                                                              float ws1, float ws2, float4* __restrict__ out,
+                                                              int by0) {
+  composite_block<IDX, false>(m, cc, light, bg, bw, bh, ws0, ws1, ws2, out, blockIdx.x, by0 + blockIdx.y, threadIdx.x);
+}
+
+// What the CTAs of the cluster wrote before it is seen by all of them after it.
+__device__ __forceinline__ void cluster_barrier() {
+  asm volatile("barrier.cluster.arrive.release;\nbarrier.cluster.wait.acquire;" ::: "memory");
+}
+
+// Colours, pyramid and composite of a small world in one launch: one cluster, whose barriers stand
+// between the steps.  A CTA takes blockDim.x / 256 of the blocks of 64 x 16 cells.  The three
+// launches that it replaces are bound by their launching and by each other's ends (us, three / one
+// launch: frame, light and image of one of three worlds in turn, and of one waited for; 64 x 64 11.3 / 8.2,
+// 30.8 / 24.4; 128 x 128 12.0 / 8.1, 31.7 / 25.6; 180 x 180 11.9 / 8.8, 31.3 / 29.4).  Up to 48 blocks, three to
+// a CTA: with four, 256 x 256, the wait is the longer one (30.4 / 31.6).
+constexpr int kImageCtas = 16;  // beyond the portable 8: half as many blocks to a CTA
+__global__ void __launch_bounds__(768) se_image_kernel(const uint32_t* __restrict__ grid,
+                                                        const float* __restrict__ noise, float4* color,
+                                                        const MipLevels mip, const RenderMat* __restrict__ mats,
+                                                        int nmat, const CompositeSrc m, const CompositeCoords cc,
+                                                        const float4* __restrict__ light, const float4* __restrict__ bg,
+                                                        int bw, int bh, float ws0, float ws1, float ws2,
+                                                        float4* __restrict__ out) {
+  __shared__ float s3[3][2][8];
+  const int sub = threadIdx.x >> 8, t = threadIdx.x & 255, b = blockIdx.x * (blockDim.x >> 8) + sub;
+  const int nbx = (m.w + 63) / 64, bx = b % nbx, by = b / nbx;
+  color_mip_block(grid, noise, color, mip, m.w, m.h, mats, nmat, bx, by, t, s3[sub]);
+  cluster_barrier();
+  if (mip.levels > 5) {
+    if (blockIdx.x == 0) mip_tail<true>(mip, threadIdx.x);  // at most 48 texels of level 6
+    cluster_barrier();
+  }
+  composite_block<uint32_t, true>(m, cc, light, bg, bw, bh, ws0, ws1, ws2, out, bx, by, t);
 }
 
 // Launches fn(by0, n) for the row blocks [by0, by0 + n) of a 2D grid, n <= 65535.
@@ -695,6 +755,30 @@ cudaError_t render_composite(const CompositeSrc& src, const CompositeCoords& coo
                                                       out, by0);
   });
   return cudaGetLastError();
+}
+
+bool image_in_one_launch(int W, int H) { return (long long)((W + 63) / 64) * ((H + 15) / 16) <= 3 * kImageCtas; }
+
+cudaError_t render_image(const uint32_t* grid, const float* noise, float4* color, const MipLevels& mip,
+                         const RenderMat* mats, int nmat, const CompositeSrc& src, const CompositeCoords& coords,
+                         const float4* light, const float4* bg, int bw, int bh, const float w_side[3], float4* out,
+                         cudaStream_t s) {
+  const int blocks = ((src.w + 63) / 64) * ((src.h + 15) / 16), sub = (blocks + kImageCtas - 1) / kImageCtas;
+  static const cudaError_t allowed =
+      cudaFuncSetAttribute(se_image_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+  if (allowed != cudaSuccess) return allowed;
+  cudaLaunchConfig_t c{};
+  c.gridDim = dim3((unsigned)((blocks + sub - 1) / sub));
+  c.blockDim = dim3((unsigned)(256 * sub));
+  c.stream = s;
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeClusterDimension;
+  at.val.clusterDim.x = c.gridDim.x;
+  at.val.clusterDim.y = at.val.clusterDim.z = 1;
+  c.attrs = &at;
+  c.numAttrs = 1;
+  return cudaLaunchKernelEx(&c, se_image_kernel, grid, noise, color, mip, mats, nmat, src, coords, light, bg, bw, bh,
+                            w_side[0], w_side[1], w_side[2], out);
 }
 
 cudaError_t render_noise(float* noise, int W, int H, cudaStream_t s) {

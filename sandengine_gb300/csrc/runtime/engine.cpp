@@ -458,8 +458,7 @@ Status World::light_frame() {
   return Status::Ok();
 }
 
-Status World::render_color(const MipLevels* mip) {
-  TraceRange trace("se_world_render_color");
+Status World::ensure_color() {
   if (halo >= 0) return {SE_ERR_INVALID_ARGUMENT, "colours are rendered for whole worlds"};
   if (!d_noise) {
     cudaError_t e = cudaMalloc(&d_noise, (size_t)W * H * sizeof(float));
@@ -470,9 +469,16 @@ Status World::render_color(const MipLevels* mip) {
     cudaError_t e = cudaMalloc(&d_color, (size_t)W * H * sizeof(float4));
     if (e != cudaSuccess) return {SE_ERR_OUT_OF_MEMORY, std::string("cudaMalloc: ") + cudaGetErrorString(e)};
   }
+  return Status::Ok();
+}
+
+Status World::render_color(const MipLevels* mip) {
+  TraceRange trace("se_world_render_color");
+  Status s = ensure_color();
+  if (!s.ok()) return s;
   Timed* t = nullptr;
   if (timing) {
-    Status s = timing_begin(2, (long long)W * H, 1, &t);
+    s = timing_begin(2, (long long)W * H, 1, &t);
     if (!s.ok()) return s;
   }
   if (mip)
@@ -504,7 +510,9 @@ Status World::composite(const float* bg, int bw, int bh) {
     mips.push_back(m);
   }
   for (int l = 1; l < n; ++l) mip.level[l] = mips[(size_t)l - 1];
-  Status s = render_color(&mip);  // colours and the pyramid in one pass
+  // a small world's image is one launch, unless its passes are to be timed one by one
+  const bool one = n > 1 && !timing && image_in_one_launch(W, H);
+  Status s = one ? ensure_color() : render_color(&mip);  // colours and the pyramid in one pass
   if (!s.ok()) return s;
   if (n == 1)
     SE_CUDA(cudaMemcpyAsync(mips[0], &d_color->w, sizeof(float), cudaMemcpyDeviceToDevice, stream));
@@ -540,6 +548,11 @@ Status World::composite(const float* bg, int bw, int bh) {
     cudaError_t e = cudaMalloc(&d_coords, composite_coords_bytes(W, H));
     if (e != cudaSuccess) return {SE_ERR_OUT_OF_MEMORY, std::string("cudaMalloc: ") + cudaGetErrorString(e)};
     SE_CUDA(render_composite_coords(d_coords, src, &coords, stream));
+  }
+  if (one) {
+    SE_CUDA(render_image(buf[cur], d_noise, d_color, mip, rs->d_render, rs->num_materials(), src, coords,
+                         light[0] ? light[lcur] : nullptr, bgd, bw, bh, kBlurSideWeight, d_composite, stream));
+    return Status::Ok();
   }
   Timed* t = nullptr;
   if (timing) {

@@ -34,6 +34,27 @@ def test_light_and_composite_match_port(se, rulesets, ports, shape):
     assert np.array_equal(sim.output_color.view(np.uint32), col.view(np.uint32))
 
 
+@pytest.mark.parametrize("shape", [(2, 1), (1, 2), (64, 64), (256, 192), (257, 192), (256, 193), (64, 768), (64, 769),
+                                   (3072, 16), (3073, 16), (1, 768), (768, 1), (191, 255)])
+def test_image_in_one_launch_matches_port(se, rulesets, ports, shape):
+    """Worlds of up to 48 blocks of 64 x 16 cells have their image made by one cluster; timed
+    passes are launched one by one.  Both with a background, against the oracle port."""
+    W, H = shape
+    P = ports["twelve_materials"]
+    sim = se.Simulation(se.parse_string(rulesets["twelve_materials"]), (W, H))
+    g = wl.patch_fill(W, H, 6, *wl.twelve_fill_spec(), patch=8)
+    sim.grid = g
+    sim.params.frame = 3
+    bg = np.random.default_rng(3).random((5, 7, 4), dtype=np.float32)
+    sim.set_light(True)
+    light = np.random.default_rng(4).random((H, W, 4), dtype=np.float32)
+    sim.output_light = light
+    want = P.composite(P.color(g), light, bg)
+    for timing in (False, True):
+        sim.set_timing(timing)
+        assert np.array_equal(sim.composite(bg).view(np.uint32), want.view(np.uint32))
+
+
 @pytest.mark.parametrize("shape", [(97, 70), (1, 100), (100, 1), (32, 32), (33, 31), (2000, 3), (1048576, 1),
                                    (3, 1048575), (1048573, 2)])
 def test_colour_noise_matches_port(se, rulesets, ports, shape):
