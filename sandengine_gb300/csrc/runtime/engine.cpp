@@ -189,8 +189,12 @@ Status World::autotune(int reps, int* best_k) {
   SE_CUDA(cudaEventCreate(&b));
   double best_multi = 0, best_one = 0;
   const TileVariant *vm = nullptr, *v1 = nullptr;
+  const LutShape lut = rs->lut_shape();
+  int dev = 0, sms = 1;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   for (const TileVariant& v : tile_variants()) {
-    if (!v.tuned(rs->lut_shape(), (long long)W * H)) continue;
+    if (!v.tuned(lut, (long long)W * H)) continue;
     Status s = launch_tiles(f0, v.kmax, &v, false);  // warm-up
     if (!s.ok()) return s;
     SE_CUDA(cudaEventRecord(a, stream));
@@ -202,7 +206,17 @@ Status World::autotune(int reps, int* best_k) {
     SE_CUDA(cudaEventSynchronize(b));
     float ms = 0;
     SE_CUDA(cudaEventElapsedTime(&ms, a, b));
-    const double rate = (double)W * H * v.kmax * reps / (ms > 0 ? ms : 1e-6);  // cell updates per ms
+    double rate = (double)W * H * v.kmax * reps / (ms > 0 ? ms : 1e-6);  // cell updates per ms
+    if (lut.nib_entries) {
+      // Among shapes that take about as long, the one that updates fewer halo cells leaves more of
+      // the chip to other streams, the more so the more of it a launch fills (us of 60 frames, three
+      // worlds in turn / one waited for; four materials 4096^2 112x112 363 / 477, 240x176 314 / 445; twelve
+      // 6000x5000 925 / 1121, 240x240 752 / 1134; twelve 2048^2 48x48 168 / 274, 112x112 136 / 277).
+      const long long ctas = (long long)((W + v.tw - 1) / v.tw) * ((H + v.th - 1) / v.th);
+      const double fill = std::min(1.0, (double)ctas * v.nt / (1024.0 * sms));
+      const double cells = (double)v.sw() * v.sh() / ((double)v.tw * v.th);  // updated per cell kept
+      rate /= 1.0 + 0.6 * fill * fill * (cells - 1.0);
+    }
     if (v.kmax == 1 && rate > best_one) best_one = rate, v1 = &v;
     if (rate > best_multi) best_multi = rate, vm = &v;
   }
