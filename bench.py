@@ -315,7 +315,7 @@ def run_ours(args, rep):
     def one_step(r):
         sim.run_frames(FRAMES_PER_STEP, mods[r])
         if args.light:
-            sim.composite_device()  # colour render, its pyramid and the composite
+            sim.composite_device()  # the pyramid and the composite
 
     for r in range(args.warmup):
         one_step(r)
@@ -414,9 +414,9 @@ def run_ours(args, rep):
         "clocks": clocks.summary(),
     }
     # algorithmic bytes per cell: light = old id, new id, old light in, light out (4 + 4 + 16 + 16);
-    # colour (inside the composite) = id, noise, RGBA out and a quarter of the level-1 alpha
-    # float; composite = colour, light, RGBA out (the smaller pyramid levels are not counted)
-    for p, name, bpc in ((1, "light_pass", 40.0), (2, "color_pass", 25.0), (3, "composite_pass", 48.0)):
+    # the composite's pyramid = id and a quarter of the level-1 alpha float; composite = id,
+    # noise, light, RGBA out (the smaller pyramid levels are not counted)
+    for p, name, bpc in ((1, "light_pass", 40.0), (2, "pyramid_pass", 5.0), (3, "composite_pass", 40.0)):
         if p in passes and passes[p]["launches"]:
             t = passes[p]
             avg_s = t["kernel_ms"] / t["launches"] / 1e3
@@ -426,7 +426,7 @@ def run_ours(args, rep):
                          "share_of_step": t["kernel_ms"] / ms if ms else None}
     if args.light:
         out["config"]["workload"] += ("; light field kept (light pass after every frame), one headless composite "
-                                      "(colour render, pyramid, composite) per step")
+                                      "(pyramid, composite) per step")
     if e2e:
         out["e2e"] = e2e
     if spec["name"] == "world16384" and not args.light and not args.k and not args.tile:

@@ -262,8 +262,9 @@ int se_world_read_timing(se_world* w, double* kernel_ms, long long* launches, lo
  * does).  The roofline of one fusion depth, e.g. the k = 8 launches of 60-frame steps. */
 int se_world_peek_timing_frames(se_world* w, int frames, double* kernel_ms, long long* launches);
 /* The same for the light pass (pass = 1; algorithmic bytes 40 x cells: old and new id, old
- * and new RGBA32F light), the colour pass (pass = 2; 24 x cells: id, noise, RGBA32F) and the
- * composite (pass = 3; 48 x cells: colour, light, output; its pyramid is not timed). */
+ * and new RGBA32F light), the colour pass (pass = 2; 24 x cells: id, noise, RGBA32F; a composite's
+ * pyramid counts here too, 5 x cells: id, a quarter of the level-1 alpha) and the composite (pass = 3;
+ * 40 x cells: id, noise, light, output). */
 int se_world_read_pass_timing(se_world* w, int pass, double* kernel_ms, long long* launches, long long* cells);
 
 /* ---- many worlds (no counterpart in the reference, which runs one world) --------------- */

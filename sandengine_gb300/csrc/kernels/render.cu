@@ -197,20 +197,23 @@ __device__ __forceinline__ float mip_texel(float a, float b, float c, float d, i
   return fmul(fadd(fadd(fadd(a, b), c), d), 0.25f);
 }
 
-// Colours and levels 1 to 4 of the alpha pyramid in one pass: a cell's alpha is its material's,
-// so level 1 comes from the same cells.  A thread takes 2 x 2 cells (a texel of level 1), a
-// warp 16 x 8 cells, whose texels of levels 2 and 3 it reduces by shuffles, and a CTA 64 x 16,
-// whose texels of level 4 need one barrier; se_mip_tail_kernel makes levels 5 and 6 (no larger
-// lod is sampled).  A launch per level cost 3-4 us each: 1920 x 1080 12.4 + 29 -> 16.4 us, 64 x 64
-// 4.1 + 11.4 -> 7.2, 4096 x 4096 66 + 39 -> 78, 8192 x 8192 250 + 54 -> 283.  64 x 64 cells a CTA with
-// all six levels reduced in shared memory kept too few loads in flight between its barriers
-// (8192 x 8192: 323 and 545 us with 256 and 1024 threads).
+__device__ __forceinline__ float cell_alpha(uint32_t id, const RenderMat* __restrict__ mats, int nmat) {
+  return __ldg(&mats[mat_index(id, nmat)].color[3]);
+}
+
+// Levels 1 to 4 of the alpha pyramid in one pass over the ids: a cell's alpha is its material's.
+// A thread takes 2 x 2 cells (a texel of level 1), a warp 16 x 8 cells, whose texels of levels 2 and 3
+// it reduces by shuffles, and a CTA 64 x 16, whose texels of level 4 need one barrier;
+// se_mip_tail_kernel makes levels 5 and 6 (no larger lod is sampled).  A launch per level cost 3-4 us
+// each; with the colours written in the same pass 1920 x 1080 takes 20.4 us and 8192 x 8192 279, the
+// pyramid alone (both kernels) 12.2 and 135.  64 x 64 cells a CTA with all six levels reduced in shared memory kept
+// too few loads in flight between its barriers (8192 x 8192 with colours: 323 and 545 us with 256 and 1024
+// threads, 283 so).
 // Block (bx, by) of 64 x 16 cells by threads t = 0 .. 255 (whole CTAs take part; blocks beyond the world
 // write nothing).
-__device__ __forceinline__ void color_mip_block(const uint32_t* __restrict__ grid, const float* __restrict__ noise,
-                                                float4* out, const MipLevels& mip, int W, int H,
-                                                const RenderMat* __restrict__ mats, int nmat, int bx, int by, int t,
-                                                float (*s3)[8]) {
+__device__ __forceinline__ void mip_block(const uint32_t* __restrict__ grid, const MipLevels& mip, int W, int H,
+                                          const RenderMat* __restrict__ mats, int nmat, int bx, int by, int t,
+                                          float (*s3)[8]) {
   const int lane = t & 31, wx = (t >> 5) & 3, wy = t >> 7;
   const int x = bx * 32 + wx * 8 + (lane & 7), y = by * 8 + wy * 4 + (lane >> 3);
   const int c0 = 2 * x, r0 = 2 * y;
@@ -223,24 +226,17 @@ __device__ __forceinline__ void color_mip_block(const uint32_t* __restrict__ gri
       const int r = min(r0 + dr, H - 1);  // at an odd last row or column the pair's second index is clamped
       const size_t i = (size_t)r * W + c0;
       uint32_t id0, id1;
-      float n0, n1;
       if (pair && (W & 1) == 0) {  // 8-byte aligned pairs
         const uint2 g = __ldg(reinterpret_cast<const uint2*>(grid + i));
-        const float2 z = __ldg(reinterpret_cast<const float2*>(noise + i));
-        id0 = g.x, id1 = g.y, n0 = z.x, n1 = z.y;
+        id0 = g.x, id1 = g.y;
       } else {
-        id0 = __ldg(grid + i), n0 = __ldg(noise + i);
+        id0 = __ldg(grid + i);
         id1 = pair ? __ldg(grid + i + 1) : id0;
-        n1 = pair ? __ldg(noise + i + 1) : n0;
       }
-      const float4 k0 = cell_color(id0, n0, mats, nmat), k1 = cell_color(id1, n1, mats, nmat);
-      if (r == r0 + dr) {
-        out[i] = k0;
-        if (pair) out[i + 1] = k1;
-      }
-      a[dr][0] = k0.w;
-      a[dr][1] = k1.w;
+      a[dr][0] = cell_alpha(id0, mats, nmat);
+      a[dr][1] = cell_alpha(id1, mats, nmat);
     }
+    if (mip.levels == 1) mip.level[1][0] = a[0][0];  // one cell
     v = fmul(fadd(fadd(fadd(a[0][0], a[0][1]), a[1][0]), a[1][1]), 0.25f);
     if (mip.levels > 1 && x < mip.w[1] && y < mip.h[1]) mip.level[1][(size_t)y * mip.w[1] + x] = v;
   }
@@ -266,12 +262,10 @@ __device__ __forceinline__ void color_mip_block(const uint32_t* __restrict__ gri
   }
 }
 
-__global__ void __launch_bounds__(256) se_color_mip_kernel(const uint32_t* __restrict__ grid,
-                                                           const float* __restrict__ noise, float4* __restrict__ out,
-                                                           const MipLevels mip, int W, int H,
-                                                           const RenderMat* __restrict__ mats, int nmat, int by0) {
+__global__ void __launch_bounds__(256) se_mip_kernel(const uint32_t* __restrict__ grid, const MipLevels mip, int W,
+                                                     int H, const RenderMat* __restrict__ mats, int nmat, int by0) {
   __shared__ float s3[2][8];
-  color_mip_block(grid, noise, out, mip, W, H, mats, nmat, blockIdx.x, by0 + blockIdx.y, threadIdx.x, s3);
+  mip_block(grid, mip, W, H, mats, nmat, blockIdx.x, by0 + blockIdx.y, threadIdx.x, s3);
 }
 
 // A load: of what an earlier launch wrote, or (SAME) this launch itself, before a barrier.
@@ -543,7 +537,7 @@ __device__ __forceinline__ Shared shared_terms(const CompositeSrc& m, const Comp
   // seven distinct samples.  lod 0 is a magnification (level 0, nearest); lod l >= 1 reads
   // the alpha level in slot l, bilinearly.
   float s[kOccLods];
-  s[0] = load<SAME>(&m.color[(IDX)__ldg(cc.nrow + r0) * (IDX)m.w + (IDX)__ldg(cc.ncol + k)].w);
+  s[0] = cell_alpha(__ldg(m.grid + ((IDX)__ldg(cc.nrow + r0) * (IDX)m.w + (IDX)__ldg(cc.ncol + k))), m.mats, m.nmat);
 #pragma unroll
   for (int l = 1; l < kOccLods; ++l) {
     const Taps c = load_taps(cc.col + (size_t)l * cc.lw + k), r = load_taps(cc.row + (size_t)l * cc.lh + r0);
@@ -594,9 +588,10 @@ __global__ void __launch_bounds__(256) se_composite_coords_kernel(CompositeTable
 // terms are computed per row (the choice is uniform in a warp).  The taps of every column pair and
 // row along every sampled texture, their indices wrapped, come from tables made once per world: a
 // sample is then two 16-byte loads, four taps and its weights, without the index arithmetic and
-// the wrap branch of its own.  Bound by the latency of its ~32 taps at 32 warps an SM (1920 x 1080:
-// 14.1 M warp instructions instead of 17.8 M, 36.6 -> 27.1 us; 64 x 64 8.3 -> 4.3, 4096 x 4096
-// 181 -> 155 us = 5.2 TB/s of 48 B a pixel).  Tables rebuilt per CTA in shared memory cost what they
+// the wrap branch of its own.  Bound by the latency of its ~32 taps at 32 warps an SM (with
+// the tables 14.1 M warp instructions at 1920 x 1080 instead of 17.8 M, 36.6 -> 27.1 us).  Colours are made
+// from ids and noise as they are needed, 40 B a pixel: reading a stored colour field took 32.7 us where
+// this takes 30.6 (4096 x 4096 162 / 156, 8192 x 8192 604 / 588) and the field's own pass 8-144 us more.  Tables rebuilt per CTA in shared memory cost what they
 // saved (35 and 189 us), as did one lane per pixel with the shared terms passed by shuffles.
 template <class IDX, bool SAME>
 __device__ __forceinline__ void composite_block(const CompositeSrc& m, const CompositeCoords& cc,
@@ -614,12 +609,14 @@ __device__ __forceinline__ void composite_block(const CompositeSrc& m, const Com
   const float2 pvs = __ldg(reinterpret_cast<const float2*>(cc.pv + r0));
   // texture(color_tex, uv, 0.0): a magnification, the nearest texel
   const bool two = c0 + 1 < W, down = r0 + 1 < H;
-  float4 cols[2][2];
+  uint32_t ids[2][2];
+  float nz[2][2];
 #pragma unroll
   for (int dr = 0; dr < 2; ++dr) {
     const IDX p = (IDX)(dr && down ? iys.y : iys.x) * (IDX)W;
-    cols[dr][0] = load<SAME>(m.color + (p + (IDX)ixs.x));
-    cols[dr][1] = load<SAME>(m.color + (p + (IDX)(two ? ixs.y : ixs.x)));
+    const IDX i0 = p + (IDX)ixs.x, i1 = p + (IDX)(two ? ixs.y : ixs.x);
+    ids[dr][0] = __ldg(m.grid + i0), nz[dr][0] = __ldg(m.noise + i0);
+    ids[dr][1] = __ldg(m.grid + i1), nz[dr][1] = __ldg(m.noise + i1);
   }
   const float ambient = 0.1f;
   Shared S = shared_terms<IDX, SAME>(m, cc, light, k, r0, ws0, ws1, ws2);
@@ -638,7 +635,7 @@ __device__ __forceinline__ void composite_block(const CompositeSrc& m, const Com
       const int cx = c0 + dc;
       if (cx >= W) break;
       const float u = dc ? us.y : us.x;
-      float4 col = cols[dr][dc];
+      float4 col = cell_color(ids[dr][dc], nz[dr][dc], m.mats, m.nmat);
       col.x = gclamp(fmul(col.x, shade), 0.0f, 1.0f);
       col.y = gclamp(fmul(col.y, shade), 0.0f, 1.0f);
       col.z = gclamp(fmul(col.z, shade), 0.0f, 1.0f);
@@ -668,24 +665,21 @@ __device__ __forceinline__ void cluster_barrier() {
   asm volatile("barrier.cluster.arrive.release;\nbarrier.cluster.wait.acquire;" ::: "memory");
 }
 
-// Colours, pyramid and composite of a small world in one launch: one cluster, whose barriers stand
+// Pyramid and composite of a small world in one launch: one cluster, whose barriers stand
 // between the steps.  A CTA takes blockDim.x / 256 of the blocks of 64 x 16 cells.  The three
 // launches that it replaces are bound by their launching and by each other's ends (us, three / one
 // launch: frame, light and image of one of three worlds in turn, and of one waited for; 64 x 64 11.3 / 8.2,
 // 30.8 / 24.4; 128 x 128 12.0 / 8.1, 31.7 / 25.6; 180 x 180 11.9 / 8.8, 31.3 / 29.4).  Up to 48 blocks, three to
 // a CTA: with four, 256 x 256, the wait is the longer one (30.4 / 31.6).
 constexpr int kImageCtas = 16;  // beyond the portable 8: half as many blocks to a CTA
-__global__ void __launch_bounds__(768) se_image_kernel(const uint32_t* __restrict__ grid,
-                                                        const float* __restrict__ noise, float4* color,
-                                                        const MipLevels mip, const RenderMat* __restrict__ mats,
-                                                        int nmat, const CompositeSrc m, const CompositeCoords cc,
-                                                        const float4* __restrict__ light, const float4* __restrict__ bg,
-                                                        int bw, int bh, float ws0, float ws1, float ws2,
-                                                        float4* __restrict__ out) {
+__global__ void __launch_bounds__(768) se_image_kernel(const MipLevels mip, const CompositeSrc m,
+                                                       const CompositeCoords cc, const float4* __restrict__ light,
+                                                       const float4* __restrict__ bg, int bw, int bh, float ws0,
+                                                       float ws1, float ws2, float4* __restrict__ out) {
   __shared__ float s3[3][2][8];
   const int sub = threadIdx.x >> 8, t = threadIdx.x & 255, b = blockIdx.x * (blockDim.x >> 8) + sub;
   const int nbx = (m.w + 63) / 64, bx = b % nbx, by = b / nbx;
-  color_mip_block(grid, noise, color, mip, m.w, m.h, mats, nmat, bx, by, t, s3[sub]);
+  mip_block(m.grid, mip, m.w, m.h, m.mats, m.nmat, bx, by, t, s3[sub]);
   cluster_barrier();
   if (mip.levels > 5) {
     if (blockIdx.x == 0) mip_tail<true>(mip, threadIdx.x);  // at most 48 texels of level 6
@@ -702,11 +696,10 @@ void for_row_blocks(int blocks, F&& fn) {
 
 }  // namespace
 
-cudaError_t render_color_mip(const uint32_t* grid, const float* noise, float4* out, const MipLevels& mip, int W, int H,
-                             const RenderMat* mats, int nmat, cudaStream_t s) {
+cudaError_t render_mips(const uint32_t* grid, const MipLevels& mip, int W, int H, const RenderMat* mats, int nmat,
+                        cudaStream_t s) {
   for_row_blocks((H + 15) / 16, [&](int by0, unsigned n) {
-    se_color_mip_kernel<<<dim3((unsigned)((W + 63) / 64), n), 256, 0, s>>>(grid, noise, out, mip, W, H, mats, nmat,
-                                                                           by0);
+    se_mip_kernel<<<dim3((unsigned)((W + 63) / 64), n), 256, 0, s>>>(grid, mip, W, H, mats, nmat, by0);
   });
   if (mip.levels > 5) {
     const long long n = (long long)((mip.w[5] + 1) / 2) * ((mip.h[5] + 1) / 2);
@@ -759,8 +752,7 @@ cudaError_t render_composite(const CompositeSrc& src, const CompositeCoords& coo
 
 bool image_in_one_launch(int W, int H) { return (long long)((W + 63) / 64) * ((H + 15) / 16) <= 3 * kImageCtas; }
 
-cudaError_t render_image(const uint32_t* grid, const float* noise, float4* color, const MipLevels& mip,
-                         const RenderMat* mats, int nmat, const CompositeSrc& src, const CompositeCoords& coords,
+cudaError_t render_image(const MipLevels& mip, const CompositeSrc& src, const CompositeCoords& coords,
                          const float4* light, const float4* bg, int bw, int bh, const float w_side[3], float4* out,
                          cudaStream_t s) {
   const int blocks = ((src.w + 63) / 64) * ((src.h + 15) / 16), sub = (blocks + kImageCtas - 1) / kImageCtas;
@@ -777,8 +769,8 @@ cudaError_t render_image(const uint32_t* grid, const float* noise, float4* color
   at.val.clusterDim.y = at.val.clusterDim.z = 1;
   c.attrs = &at;
   c.numAttrs = 1;
-  return cudaLaunchKernelEx(&c, se_image_kernel, grid, noise, color, mip, mats, nmat, src, coords, light, bg, bw, bh,
-                            w_side[0], w_side[1], w_side[2], out);
+  return cudaLaunchKernelEx(&c, se_image_kernel, mip, src, coords, light, bg, bw, bh, w_side[0], w_side[1], w_side[2],
+                            out);
 }
 
 cudaError_t render_noise(float* noise, int W, int H, cudaStream_t s) {

@@ -32,7 +32,8 @@ cudaError_t light_pass(const uint32_t* old_grid, const uint32_t* new_grid, const
                        int W, int H, const RenderMat* mats, int nmat, cudaStream_t s);
 
 // Headless composite (shaders/fragment140.glsl:70-100): the colour field's box-filter
-// pyramid, then one RGBA32F pixel per texel.  GL filtering is fixed to the spec's formulas
+// pyramid, then one RGBA32F pixel per texel.  The colour field itself is not stored: a texel is
+// its cell's id and noise (8 bytes instead of 16 written and 16 read).  GL filtering is fixed to the spec's formulas
 // in binary32 (mirrored-repeat wrap, nearest / bilinear taps, LINEAR_MIPMAP_NEAREST level
 // choice); the three blur weights exp(-gamma) for gamma 0.5, 0.35, 0.2 are passed in.
 // The fragment reads levels above 0 only through their alpha (the occlusion's
@@ -40,12 +41,15 @@ cudaError_t light_pass(const uint32_t* old_grid, const uint32_t* new_grid, const
 // the alpha channel, a quarter of the bytes.
 // The occlusion's textureLod calls use the integer lods 0 .. 6.
 constexpr int kOccLods = 7;
-// What the composite samples: the colour field (level 0) and, for lod l = 1 .. 6, the alpha
+// What the composite samples: the colour field (level 0), by ids and noise, and, for lod l = 1 .. 6, the alpha
 // level textureLod reads at lod l.  With LINEAR_MIPMAP_NEAREST that is level
 // ceil(l + 0.5) - 1 = l, or the last level of a shorter pyramid; a 1 x 1 field has no level
 // 1, and its slots hold a copy of its own alpha.
 struct CompositeSrc {
-  const float4* color;
+  const uint32_t* grid;
+  const float* noise;
+  const RenderMat* mats;
+  int nmat;
   int w, h;
   const float* alpha[kOccLods];  // [0] is unused
   int aw[kOccLods], ah[kOccLods];
@@ -60,11 +64,9 @@ struct MipLevels {
   int w[kOccLods], h[kOccLods];
   int levels;
 };
-// output_color as render_color, plus the pyramid's alpha levels (mip.levels <= 1: none): a
-// cell's alpha is its material's colour alpha, so they come from the same pass instead of a
-// second read of the RGBA field.
-cudaError_t render_color_mip(const uint32_t* grid, const float* noise, float4* out, const MipLevels& mip, int W, int H,
-                             const RenderMat* mats, int nmat, cudaStream_t s);
+// The pyramid's alpha levels of a grid; levels == 1 (a single cell): its alpha in level[1].
+cudaError_t render_mips(const uint32_t* grid, const MipLevels& mip, int W, int H, const RenderMat* mats, int nmat,
+                        cudaStream_t s);
 // A coordinate's two bilinear taps along one axis of a texture: the wrapped indices, and the
 // weights of the second and of the first.
 struct alignas(16) Taps {
@@ -104,10 +106,9 @@ size_t composite_coords_bytes(int W, int H);
 cudaError_t render_composite_coords(void* buf, const CompositeSrc& src, CompositeCoords* out, cudaStream_t s);
 cudaError_t render_composite(const CompositeSrc& src, const CompositeCoords& coords, const float4* light,
                              const float4* bg, int bw, int bh, const float w_side[3], float4* out, cudaStream_t s);
-// Small worlds: render_color_mip and render_composite in one launch.
+// Small worlds: render_mips and render_composite in one launch.
 bool image_in_one_launch(int W, int H);
-cudaError_t render_image(const uint32_t* grid, const float* noise, float4* color, const MipLevels& mip,
-                         const RenderMat* mats, int nmat, const CompositeSrc& src, const CompositeCoords& coords,
+cudaError_t render_image(const MipLevels& mip, const CompositeSrc& src, const CompositeCoords& coords,
                          const float4* light, const float4* bg, int bw, int bh, const float w_side[3], float4* out,
                          cudaStream_t s);
 

@@ -472,33 +472,30 @@ Status World::light_frame() {
   return Status::Ok();
 }
 
-Status World::ensure_color() {
+Status World::ensure_noise() {
   if (halo >= 0) return {SE_ERR_INVALID_ARGUMENT, "colours are rendered for whole worlds"};
   if (!d_noise) {
     cudaError_t e = cudaMalloc(&d_noise, (size_t)W * H * sizeof(float));
     if (e != cudaSuccess) return {SE_ERR_OUT_OF_MEMORY, std::string("cudaMalloc: ") + cudaGetErrorString(e)};
     SE_CUDA(render_noise(d_noise, W, H, stream));
   }
+  return Status::Ok();
+}
+
+Status World::render_color() {
+  TraceRange trace("se_world_render_color");
+  Status s = ensure_noise();
+  if (!s.ok()) return s;
   if (!d_color) {
     cudaError_t e = cudaMalloc(&d_color, (size_t)W * H * sizeof(float4));
     if (e != cudaSuccess) return {SE_ERR_OUT_OF_MEMORY, std::string("cudaMalloc: ") + cudaGetErrorString(e)};
   }
-  return Status::Ok();
-}
-
-Status World::render_color(const MipLevels* mip) {
-  TraceRange trace("se_world_render_color");
-  Status s = ensure_color();
-  if (!s.ok()) return s;
   Timed* t = nullptr;
   if (timing) {
     s = timing_begin(2, (long long)W * H, 1, &t);
     if (!s.ok()) return s;
   }
-  if (mip)
-    SE_CUDA(render_color_mip(buf[cur], d_noise, d_color, *mip, W, H, rs->d_render, rs->num_materials(), stream));
-  else
-    SE_CUDA(se::rt::render_color(buf[cur], d_noise, d_color, W, H, rs->d_render, rs->num_materials(), stream));
+  SE_CUDA(se::rt::render_color(buf[cur], d_noise, d_color, W, H, rs->d_render, rs->num_materials(), stream));
   if (t) SE_CUDA(cudaEventRecord(t->b, stream));
   return Status::Ok();
 }
@@ -523,15 +520,16 @@ Status World::composite(const float* bg, int bw, int bh) {
     if (e != cudaSuccess) return {SE_ERR_OUT_OF_MEMORY, std::string("cudaMalloc: ") + cudaGetErrorString(e)};
     mips.push_back(m);
   }
-  for (int l = 1; l < n; ++l) mip.level[l] = mips[(size_t)l - 1];
+  for (int l = 1; l < std::max(n, 2); ++l) mip.level[l] = mips[(size_t)l - 1];
   // a small world's image is one launch, unless its passes are to be timed one by one
-  const bool one = n > 1 && !timing && image_in_one_launch(W, H);
-  Status s = one ? ensure_color() : render_color(&mip);  // colours and the pyramid in one pass
+  const bool one = !timing && image_in_one_launch(W, H);
+  Status s = ensure_noise();
   if (!s.ok()) return s;
-  if (n == 1)
-    SE_CUDA(cudaMemcpyAsync(mips[0], &d_color->w, sizeof(float), cudaMemcpyDeviceToDevice, stream));
   CompositeSrc src{};
-  src.color = d_color;
+  src.grid = buf[cur];
+  src.noise = d_noise;
+  src.mats = rs->d_render;
+  src.nmat = rs->num_materials();
   src.w = W;
   src.h = H;
   for (int l = 1; l < kOccLods; ++l) {
@@ -564,11 +562,17 @@ Status World::composite(const float* bg, int bw, int bh) {
     SE_CUDA(render_composite_coords(d_coords, src, &coords, stream));
   }
   if (one) {
-    SE_CUDA(render_image(buf[cur], d_noise, d_color, mip, rs->d_render, rs->num_materials(), src, coords,
-                         light[0] ? light[lcur] : nullptr, bgd, bw, bh, kBlurSideWeight, d_composite, stream));
+    SE_CUDA(render_image(mip, src, coords, light[0] ? light[lcur] : nullptr, bgd, bw, bh, kBlurSideWeight, d_composite,
+                         stream));
     return Status::Ok();
   }
   Timed* t = nullptr;
+  if (timing) {
+    s = timing_begin(2, (long long)W * H, 1, &t);
+    if (!s.ok()) return s;
+  }
+  SE_CUDA(render_mips(src.grid, mip, W, H, src.mats, src.nmat, stream));
+  if (t) SE_CUDA(cudaEventRecord(t->b, stream));
   if (timing) {
     s = timing_begin(3, (long long)W * H, 1, &t);
     if (!s.ok()) return s;

@@ -133,9 +133,8 @@ struct World {
   float4* d_color = nullptr;
   Status set_light(bool on);
   Status light_frame();  // light pass for the frame just taken (old grid buf[cur ^ 1])
-  // The current grid's colours into d_color; with mip, also the pyramid's alpha levels.
-  Status ensure_color();  // the noise field and the colour buffer
-  Status render_color(const MipLevels* mip = nullptr);
+  Status ensure_noise();
+  Status render_color();  // the current grid's colours into d_color
   // Headless composite of the current grid (colour, its pyramid, the light field when
   // kept, an optional background image) into d_composite (RGBA32F per cell).
   std::vector<float*> mips;  // the colour pyramid's levels 1.. (alpha only)
