@@ -69,14 +69,19 @@ Status Server::create(std::shared_ptr<Ruleset> r, long long budget_bytes) {
 Status Server::set_frames_per_iteration(int k) {
   std::lock_guard<std::mutex> g(mu);
   if (live) return {SE_ERR_INVALID_ARGUMENT, "the frames per iteration cannot change while the server runs"};
-  // The first compiled variant with the fewest frames >= k: for k = 8 the 128x64 tiles,
-  // which serve sessions of 128-2048 cells a side best (the serving benchmark's highest
-  // throughput, 770 G cell-updates/s, against 690-734 G with 256x128, 128x128 or 256x64
-  // tiles): their smaller halo loss on the large tiles does not make up for the waste on
-  // the small sessions and the coarser work units of an iteration.
+  // The first compiled variant with the fewest frames >= k.  For k = 8 on bytes the 128x64 tiles,
+  // which serve sessions of 128-2048 cells a side best (770 G cell-updates/s against 690-734 G
+  // with 256x128, 128x128 or 256x64 tiles: a smaller halo does not make up for the waste on the small
+  // sessions and the coarser work units of an iteration); with two cells a byte 112x112, and
+  // the smaller tiles of as many frames for iterations of few cells (the loop's choice).
   const TileVariant* v = pick_variant(k, rs->lut_shape(), -1);
   if (!v || k < 1) return {SE_ERR_INVALID_ARGUMENT, "no kernel variant for this many frames per iteration"};
   variant = v;
+  small_variant = nullptr;
+  if (rs->lut_shape().nib_entries)
+    for (const TileVariant& t : tile_variants())
+      if (!small_variant && t.fits(rs->lut_shape()) && t.kmax == v->kmax && t.tw * t.th < v->tw * v->th)
+        small_variant = &t;
   return Status::Ok();
 }
 
@@ -434,8 +439,6 @@ Status Server::serve_batched(std::unique_lock<std::mutex>& lk) {
                      [&](int a, int b) { return requests[(size_t)a].arrival_ms < requests[(size_t)b].arrival_ms; });
   }
   const int K = variant->kmax;
-  const size_t smem = tile_smem_bytes(*variant, rs->lut_shape());
-  cudaKernel_t kern = rs->module->get(variant->serve_name());
   const uint16_t* lut = rs->d_lut;
   size_t next = 0;
   std::deque<int> waiting;  // sessions with queued requests, in order of their turn
@@ -535,6 +538,11 @@ Status Server::serve_batched(std::unique_lock<std::mutex>& lk) {
     if (it >= kRing) SE_CUDA(cudaEventSynchronize(stg.ev));  // at most two iterations are in flight
     Status st = stage_reserve(stg, active.size());
     if (!st.ok()) return st;
+    // Up to 2^22 active cells an iteration is the latency of its tiles (us a burst of requests,
+    // 112x112 / 48x48: 0.8 million cells 770 / 607, 2.7 million 1180 / 1090, 12.5 million 2878 / 3007).
+    long long cells = 0;
+    for (int sid : active) cells += (long long)sessions[(size_t)sid].W * sessions[(size_t)sid].H;
+    const TileVariant& v = small_variant && cells <= 1ll << 22 ? *small_variant : *variant;
     int total = 0;
     std::vector<int> ks(active.size());
     for (size_t a = 0; a < active.size(); ++a) {
@@ -544,7 +552,7 @@ Status Server::serve_batched(std::unique_lock<std::mutex>& lk) {
       ks[a] = k;
       stg.desc[a] = WorldDesc{ss.buf(0), ss.buf(1), ss.W, ss.H, ss.frame, ss.cur, k, 0};
       stg.prefix[a] = total;
-      total += ((ss.W + variant->tw - 1) / variant->tw) * ((ss.H + variant->th - 1) / variant->th);
+      total += ((ss.W + v.tw - 1) / v.tw) * ((ss.H + v.th - 1) / v.th);
     }
     stg.prefix[active.size()] = total;
     SE_CUDA(cudaMemcpyAsync(stg.d_desc, stg.desc, active.size() * sizeof(WorldDesc), cudaMemcpyHostToDevice, stream));
@@ -558,8 +566,8 @@ Status Server::serve_batched(std::unique_lock<std::mutex>& lk) {
       const int* pp = stg.d_prefix;
       int na = (int)active.size();
       void* args[] = {(void*)&dd, (void*)&pp, &na, (void*)&lut};
-      SE_CUDA(cudaLaunchKernel((const void*)kern, dim3((unsigned)total), dim3((unsigned)variant->nt), args, smem,
-                               stream));
+      SE_CUDA(cudaLaunchKernel((const void*)rs->module->get(v.serve_name()), dim3((unsigned)total),
+                               dim3((unsigned)v.nt), args, tile_smem_bytes(v, rs->lut_shape()), stream));
     }
     SE_CUDA(cudaEventRecord(stg.ev, stream));
     ++it;

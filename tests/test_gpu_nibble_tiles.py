@@ -86,3 +86,26 @@ def test_whole_worlds_match_port(se, rulesets, name):
             frames[i] += nf
             got = b.grid(i)
             assert np.array_equal(got, g), f"{name} world {sizes[i]}: {np.count_nonzero(got != g)} cells differ"
+
+
+@pytest.mark.parametrize("frames", [4, 8, 16])
+def test_serving_iterations_of_many_and_few_cells(se, rulesets, ports, frames):
+    """Iterations above 2^22 active cells and, once the large session is done, below."""
+    from sandengine_gb300 import workloads as wl
+    from sandengine_gb300.serving import Server
+    srv = Server(se.parse_string(rulesets["twelve_materials"]), 1 << 30)
+    srv.set_frames_per_iteration(frames)
+    want, jobs = [], []
+    for i, (w, h, n) in enumerate(((2050, 2049, 2 * frames + 3), (301, 203, 5 * frames + 1), (64, 64, 3 * frames))):
+        g = wl.patch_fill(w, h, i, *wl.twelve_fill_spec(), patch=16)
+        sid = srv.open_session(w, h, g, 2 + i)
+        mods = wl.circle_edits(w, h, 9, i, 3, [0, 3], rmin=1, rmax=20)
+        jobs.append((sid, n, [se.SimModification((m[0], m[1]), m[2], m[3], m[4]) for m in mods]))
+        ports["twelve_materials"].run(g, 2 + i, n, mods, nthreads=8)
+        want.append(g)
+    srv.start()
+    for r in [srv.submit(sid, n, mods) for sid, n, mods in jobs]:
+        srv.wait(r)
+    srv.stop()
+    for (sid, _, _), g in zip(jobs, want):
+        assert np.array_equal(srv.grid(sid), g)
