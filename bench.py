@@ -136,7 +136,7 @@ def load_traffic(workload_name, variant, k):
                           f"(the committed one is {vals['variant']} k={vals['k']} on {vals['workload']})")
         return float(vals["dram_bytes_per_launch"]), (f"ncu dram__bytes_read.sum + dram__bytes_write.sum of one "
                                                       f"{variant} launch at k={k} on {workload_name} "
-                                                      f"(profiles/tile_kernel_256x128_k8_world16384.md)")
+                                                      f"(profiles/tile_kernel_240x240_k8.md)")
     except (KeyError, ValueError):
         return None, None
 
@@ -397,8 +397,9 @@ def run_ours(args, rep):
                      "traffic_source": traffic_source,
                      "kernel": f"se_tile_{tile[0]}x{tile[1]}_k{tile[2]} (up to {k} frames per launch)",
                      "peak_source": peak_src,
-                     "bound_note": "issue-bound at k >= 2: the integer ALU pipe runs at 73% of its peak and DRAM "
-                                   "traffic equals the algorithmic bytes (profiles/tile_kernel_256x128_k8_world16384.md); "
+                     "bound_note": "bound on chip at k >= 2: the L1 data pipe runs at 71% and the integer ALU pipe at "
+                                   "67% of peak, and DRAM traffic equals the algorithmic bytes "
+                                   "(profiles/tile_kernel_240x240_k8.md); "
                                    "one_frame_launches gives the same kernel at one frame per launch, HBM-bound",
                      "algorithmic_bytes_per_launch": alg_bytes_per_launch,
                      "avg_launch_ms": avg_launch_s * 1e3, "launches": launches,

@@ -416,7 +416,11 @@ __device__ __forceinline__ uint32_t se_nib_pack(uint4 v) {
   return (v.x + v.y * 16u) + (v.z + v.w * 16u) * 256u;
 }
 
-// se_tile_run (margolus.cuh) on the word-packed array: the same contract.
+// se_tile_run (margolus.cuh) on the word-packed array: the same contract.  Bound by the ALU pipe
+// (four materials: 78% of peak) or by the L1 data pipe that gathers a table too large for shared memory
+// (twelve: 71%).  Against byte tiles with two hash lanes a block and lists of chunks, us of an
+// 8-frame launch on 8192^2: twelve materials 320-337 -> 271, later frames 317-330 -> 232.  Two words a
+// row per lane share the loop, the skip test and the checks over 8 blocks (one word: 333 -> 281).
 template <int TW, int TH, int KMAX, int NT>
 __device__ __forceinline__ void se_nib_run(const uint32_t* __restrict__ src, uint32_t* __restrict__ dst, int W,
                                            int H, int f0, int k, const uint16_t* __restrict__ lut, int X0, int Y0,
@@ -547,7 +551,8 @@ __device__ __forceinline__ void se_nib_world_step(uint32_t* sm, int stride, int 
 
 // se_resident's body on a word-packed array: the whole world with a WALL border of 4 columns on
 // the left, at least one on the right, and one row above and below; two words of padding per
-// row.  A world takes half a byte a cell, so worlds of up to about 450,000 cells fit a CTA.
+// row.  A world takes half a byte a cell, so worlds of up to about 450,000 cells fit a CTA.  Bound as
+// the tiles are (4096 worlds, 100 frames, on byte arrays / so: 28.5 / 23.5 ms).
 __device__ __forceinline__ void se_nib_resident(const SeWorldDesc& w, int frames, int out_flip,
                                                 const uint16_t* __restrict__ lut) {
   extern __shared__ __align__(16) uint8_t se_smem[];

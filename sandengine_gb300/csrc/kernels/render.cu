@@ -756,12 +756,13 @@ cudaError_t render_image(const MipLevels& mip, const CompositeSrc& src, const Co
                          const float4* light, const float4* bg, int bw, int bh, const float w_side[3], float4* out,
                          cudaStream_t s) {
   const int blocks = ((src.w + 63) / 64) * ((src.h + 15) / 16), sub = (blocks + kImageCtas - 1) / kImageCtas;
-  static const cudaError_t allowed =
-      cudaFuncSetAttribute(se_image_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-  if (allowed != cudaSuccess) return allowed;
   cudaLaunchConfig_t c{};
   c.gridDim = dim3((unsigned)((blocks + sub - 1) / sub));
   c.blockDim = dim3((unsigned)(256 * sub));
+  if (c.gridDim.x > 8) {  // beyond the portable cluster size; a setting of the current device's kernel
+    cudaError_t e = cudaFuncSetAttribute(se_image_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    if (e != cudaSuccess) return e;
+  }
   c.stream = s;
   cudaLaunchAttribute at{};
   at.id = cudaLaunchAttributeClusterDimension;

@@ -106,8 +106,8 @@ struct World {
   EditParams edit_params;  // the edit list of the current step's first launch (copied at launch)
   int default_k() const;
   // Opt-in per-launch CUDA-event timing (for roofline measurements) of the tile kernel
-  // (pass 0), the light pass (1), the colour pass (2) and the composite (3, its pyramid
-  // excluded).
+  // (pass 0), the light pass (1), the colour pass or a composite's pyramid (2) and the
+  // composite (3).
   bool timing = false;
   struct Timed {
     cudaEvent_t a, b;
