@@ -364,7 +364,7 @@ SE_API int se_world_set_tile(se_world* w, int tile_w, int tile_h, int k) {
   return guard([&] {
     if (!w) return fail(SE_ERR_INVALID_ARGUMENT, "null world");
     for (auto& t : se::rt::tile_variants())
-      if (t.tw == tile_w && t.th == tile_h && t.kmax == k) {
+      if (t.tw == tile_w && t.th == tile_h && t.kmax == k && t.compiled(w->w->rs->lut_shape())) {
         auto& W = *w->w;
         if (k == 1) {
           W.single = &t;

@@ -42,7 +42,7 @@ Status Ruleset::compile() {
   if (compiled) return Status::Ok();
   if (codegen_code) return {codegen_code, codegen_message};
   std::string log;
-  if (!compile_cubin(device_source(), &cubin, &log)) return {SE_ERR_COMPILE, "NVRTC: " + log};
+  if (!compile_cubin(device_source(), lut_shape().nib_entries > 0, &cubin, &log)) return {SE_ERR_COMPILE, "NVRTC: " + log};
   compiled = true;
   return Status::Ok();
 }

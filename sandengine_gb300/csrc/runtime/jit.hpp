@@ -27,6 +27,8 @@ struct TileVariant {
   enum { kByte = 1, kNibble = 2, kTuned = 4 };
   int use;  // the kinds of tile it is chosen for, and whether by the autotuner (set_tile may ask for any)
   long long min_cells = 0, max_cells = 1ll << 62;
+  // Whether the rule set's module holds it: shapes for 4-bit tiles only where there are such.
+  bool compiled(const LutShape& lut) const { return (use & kByte) || lut.nib_entries; }
   bool fits(const LutShape& lut) const { return use & (lut.nib_entries ? kNibble : kByte); }
   // Whether the autotuner tries it on `cells` cells (of one world, or of a batch's tiled worlds).
   bool tuned(const LutShape& lut, long long cells) const {
@@ -58,7 +60,7 @@ size_t tile_smem_bytes(const TileVariant& t, const LutShape& lut);
 std::string kernel_source(const std::string& generated_rules);
 
 // Compiles `src` to an sm_103a cubin (cached by content hash).  No GPU needed.
-bool compile_cubin(const std::string& src, std::string* cubin, std::string* log);
+bool compile_cubin(const std::string& src, bool parallel, std::string* cubin, std::string* log);
 
 struct Module {
   cudaLibrary_t lib = nullptr;
