@@ -34,8 +34,8 @@ def test_light_and_composite_match_port(se, rulesets, ports, shape):
     assert np.array_equal(sim.output_color.view(np.uint32), col.view(np.uint32))
 
 
-@pytest.mark.parametrize("shape", [(2, 1), (1, 2), (64, 64), (256, 192), (257, 192), (256, 193), (64, 768), (64, 769),
-                                   (3072, 16), (3073, 16), (1, 768), (768, 1), (191, 255)])
+@pytest.mark.parametrize("shape", [(1, 1), (2, 1), (1, 2), (64, 64), (256, 192), (257, 192), (256, 193), (64, 768),
+                                   (64, 769), (3072, 16), (3073, 16), (1, 768), (768, 1), (191, 255)])
 def test_image_in_one_launch_matches_port(se, rulesets, ports, shape):
     """Worlds of up to 48 blocks of 64 x 16 cells have their image made by one cluster; timed
     passes are launched one by one.  Both with a background, against the oracle port."""
