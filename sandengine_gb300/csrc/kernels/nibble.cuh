@@ -14,6 +14,9 @@
 // every constant they depend on, with the bound below which that does not hold, and hash that
 // lane; the few blocks below their bound take the full table.  So a block costs one hash lane
 // and one lookup, which does not wait for the hash.
+//
+// On the CPU the code runs with one thread per CTA and without the reduced tables, or, with
+// SE_WHOLE_WARPS, with its real thread counts and tables.
 #pragma once
 
 #ifdef SE_NIB
@@ -142,7 +145,9 @@ __device__ __forceinline__ uint32_t se_signs(uint32_t a, uint32_t b) {
 // Copies a shared reduced table into shared memory, 16 bytes a thread and step, asynchronously
 // (both ends hold whole groups of four words); se_nib_table_ready before the barrier.
 __device__ __forceinline__ void se_nib_copy_table(uint32_t* tab, const uint32_t* __restrict__ gtab, int nt) {
-#if SE_NIB_SHARED && defined(__CUDA_ARCH__)
+#if SE_NIB_SHARED && defined(SE_WHOLE_WARPS)
+  for (int i = threadIdx.x; i < ((SE_NIB_ENTRIES + 3) & ~3); i += nt) tab[i] = gtab[i];
+#elif SE_NIB_SHARED && defined(__CUDA_ARCH__)
   for (int i = threadIdx.x; i < (SE_NIB_ENTRIES + 3) / 4; i += nt)
     asm volatile("cp.async.ca.shared.global [%0], [%1], 16;" ::"r"(
                      (unsigned)__cvta_generic_to_shared(tab + 4 * i)),
@@ -366,9 +371,10 @@ __device__ __forceinline__ void se_nib_step(uint32_t* sm, bool& look, int ly0, i
   for (int it = warp; it < ITEMS; it += NW) {
     const int g = it / NSUB, q = it - g * NSUB;
     const int off = off0 + g * (2 * LY * G::STRIDE) + q * (2 * LX);
-    if (!se_check(off >= 0 && off + G::STRIDE + 2 < G::STRIDE * G::ROWS, 8u)) break;
+    // a lane whose check fails takes no chunk of its own, but the votes of its warp
+    const bool ok = se_check(off >= 0 && off + G::STRIDE + 2 < G::STRIDE * G::ROWS, 8u);
     if (look) ++seen;
-    if (se_nib_chunk<NT, OX>(sm, off, G::STRIDE, true, look, gx0 + c0 + 16 * LX * q, gy0 + r0 + 2 * LY * g,
+    if (se_nib_chunk<NT, OX>(sm, ok ? off : 0, G::STRIDE, ok, look, gx0 + c0 + 16 * LX * q, gy0 + r0 + 2 * LY * g,
                              x0 + (uint32_t)(g * LY) * 4262u + (uint32_t)(q * LX) * 7376u, W, H, edge, umask, tab,
                              gtab, lut))
       ++still;
@@ -529,7 +535,7 @@ __device__ __forceinline__ void se_nib_world_step(uint32_t* sm, int stride, int 
                                                   int ly0, int gx0, int gy0, int f, int W, int H, uint32_t umask,
                                                   const uint32_t* tab, const uint32_t* __restrict__ gtab,
                                                   const uint16_t* __restrict__ lut) {
-#if defined(__CUDA_ARCH__)
+#if defined(__CUDA_ARCH__) || defined(SE_WHOLE_WARPS)
   constexpr int NT = 32;
 #else
   constexpr int NT = 1;  // emulated: one thread per CTA
@@ -541,10 +547,10 @@ __device__ __forceinline__ void se_nib_world_step(uint32_t* sm, int stride, int 
     int j, q;
     se_divmod_rt(on ? base + lane : base, cpr, inv_cpr, j, q);
     const int row = ly0 + 2 * j, off = row * stride + 2 * q, gx = gx0 + 16 * q + OX, gy = gy0 + row;
-    if (!se_check(off >= 0 && off + stride + 2 < stride * rows, 8u)) break;
+    const bool ok = se_check(off >= 0 && off + stride + 2 < stride * rows, 8u);  // as in se_nib_step
     if (look) ++seen;
     const uint32_t x = (uint32_t)gx * 461u + (uint32_t)gy * 2131u + (uint32_t)f * 4541161u;
-    if (se_nib_chunk<NT, OX>(sm, off, stride, on, look, gx, gy, x, W, H, true, umask, tab, gtab, lut)) ++still;
+    if (se_nib_chunk<NT, OX>(sm, ok ? off : 0, stride, on && ok, look, gx, gy, x, W, H, true, umask, tab, gtab, lut)) ++still;
   }
   look = 8 * still > seen;
 }
@@ -560,7 +566,7 @@ __device__ __forceinline__ void se_nib_resident(const SeWorldDesc& w, int frames
   uint32_t* sm = reinterpret_cast<uint32_t*>(se_smem);
   const uint32_t* gtab = reinterpret_cast<const uint32_t*>(reinterpret_cast<const uint8_t*>(lut) + SE_NIB_OFF);
   uint32_t* tab = sm + ((stride * rows + 3) & ~3);
-#if defined(__CUDA_ARCH__)
+#if defined(__CUDA_ARCH__) || defined(SE_WHOLE_WARPS)
   const uint32_t umask = __ldg(gtab + SE_NIB_ENTRIES);
   se_nib_copy_table(tab, gtab, nt);
 #else
