@@ -336,7 +336,9 @@ SE_API void se_world_destroy(se_world* w) {
 SE_API int se_world_set_stream(se_world* w, void* s) {
   return guard([&] {
     if (!w) return fail(SE_ERR_INVALID_ARGUMENT, "null world");
+    const cudaStream_t was = w->w->stream;
     w->w->stream = s ? (cudaStream_t)s : w->w->own_stream;
+    if (w->w->stream != was) w->w->one_image = -1;
     return (int)SE_OK;
   });
 }

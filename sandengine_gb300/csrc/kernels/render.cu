@@ -670,7 +670,8 @@ __device__ __forceinline__ void cluster_barrier() {
 // launches that it replaces are bound by their launching and by each other's ends (us, three / one
 // launch: frame, light and image of one of three worlds in turn, and of one waited for; 64 x 64 11.3 / 8.2,
 // 30.8 / 24.4; 128 x 128 12.0 / 8.1, 31.7 / 25.6; 180 x 180 11.9 / 8.8, 31.3 / 29.4).  Up to 48 blocks, three to
-// a CTA: with four, 256 x 256, the wait is the longer one (30.4 / 31.6).
+// a CTA: with four, 256 x 256, the wait is the longer one (30.4 / 31.6).  Where the device (or the part of it
+// that the stream may use) has no room for such a cluster, the three launches stay.
 constexpr int kImageCtas = 16;  // beyond the portable 8: half as many blocks to a CTA
 __global__ void __launch_bounds__(768) se_image_kernel(const MipLevels mip, const CompositeSrc m,
                                                        const CompositeCoords cc, const float4* __restrict__ light,
@@ -750,26 +751,45 @@ cudaError_t render_composite(const CompositeSrc& src, const CompositeCoords& coo
   return cudaGetLastError();
 }
 
-bool image_in_one_launch(int W, int H) { return (long long)((W + 63) / 64) * ((H + 15) / 16) <= 3 * kImageCtas; }
+namespace {
+// The launch of se_image_kernel for a world of at most 3 * kImageCtas blocks; `at` holds its attribute.
+cudaError_t image_launch(int W, int H, cudaStream_t s, cudaLaunchConfig_t* c, cudaLaunchAttribute* at) {
+  const int blocks = ((W + 63) / 64) * ((H + 15) / 16), sub = (blocks + kImageCtas - 1) / kImageCtas;
+  *c = cudaLaunchConfig_t{};
+  c->gridDim = dim3((unsigned)((blocks + sub - 1) / sub));
+  c->blockDim = dim3((unsigned)(256 * sub));
+  c->stream = s;
+  *at = cudaLaunchAttribute{};
+  at->id = cudaLaunchAttributeClusterDimension;
+  at->val.clusterDim.x = c->gridDim.x;
+  at->val.clusterDim.y = at->val.clusterDim.z = 1;
+  c->attrs = at;
+  c->numAttrs = 1;
+  if (c->gridDim.x <= 8) return cudaSuccess;
+  // beyond the portable cluster size; a setting of the current device's kernel
+  return cudaFuncSetAttribute(se_image_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+}
+}  // namespace
+
+bool image_in_one_launch(int W, int H, cudaStream_t s) {
+  if ((long long)((W + 63) / 64) * ((H + 15) / 16) > 3 * kImageCtas) return false;
+  cudaLaunchConfig_t c;
+  cudaLaunchAttribute at;
+  int clusters = 0;
+  if (image_launch(W, H, s, &c, &at) == cudaSuccess &&
+      cudaOccupancyMaxActiveClusters(&clusters, se_image_kernel, &c) == cudaSuccess)
+    return clusters > 0;
+  cudaGetLastError();  // the answer is no, not a failure
+  return false;
+}
 
 cudaError_t render_image(const MipLevels& mip, const CompositeSrc& src, const CompositeCoords& coords,
                          const float4* light, const float4* bg, int bw, int bh, const float w_side[3], float4* out,
                          cudaStream_t s) {
-  const int blocks = ((src.w + 63) / 64) * ((src.h + 15) / 16), sub = (blocks + kImageCtas - 1) / kImageCtas;
-  cudaLaunchConfig_t c{};
-  c.gridDim = dim3((unsigned)((blocks + sub - 1) / sub));
-  c.blockDim = dim3((unsigned)(256 * sub));
-  if (c.gridDim.x > 8) {  // beyond the portable cluster size; a setting of the current device's kernel
-    cudaError_t e = cudaFuncSetAttribute(se_image_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-    if (e != cudaSuccess) return e;
-  }
-  c.stream = s;
-  cudaLaunchAttribute at{};
-  at.id = cudaLaunchAttributeClusterDimension;
-  at.val.clusterDim.x = c.gridDim.x;
-  at.val.clusterDim.y = at.val.clusterDim.z = 1;
-  c.attrs = &at;
-  c.numAttrs = 1;
+  cudaLaunchConfig_t c;
+  cudaLaunchAttribute at;
+  cudaError_t e = image_launch(src.w, src.h, s, &c, &at);
+  if (e != cudaSuccess) return e;
   return cudaLaunchKernelEx(&c, se_image_kernel, mip, src, coords, light, bg, bw, bh, w_side[0], w_side[1], w_side[2],
                             out);
 }

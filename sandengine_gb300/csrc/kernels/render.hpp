@@ -106,8 +106,9 @@ size_t composite_coords_bytes(int W, int H);
 cudaError_t render_composite_coords(void* buf, const CompositeSrc& src, CompositeCoords* out, cudaStream_t s);
 cudaError_t render_composite(const CompositeSrc& src, const CompositeCoords& coords, const float4* light,
                              const float4* bg, int bw, int bh, const float w_side[3], float4* out, cudaStream_t s);
-// Small worlds: render_mips and render_composite in one launch.
-bool image_in_one_launch(int W, int H);
+// Small worlds: render_mips and render_composite in one launch, where its cluster can run on the
+// device and stream.
+bool image_in_one_launch(int W, int H, cudaStream_t s);
 cudaError_t render_image(const MipLevels& mip, const CompositeSrc& src, const CompositeCoords& coords,
                          const float4* light, const float4* bg, int bw, int bh, const float w_side[3], float4* out,
                          cudaStream_t s);

@@ -522,7 +522,8 @@ Status World::composite(const float* bg, int bw, int bh) {
   }
   for (int l = 1; l < std::max(n, 2); ++l) mip.level[l] = mips[(size_t)l - 1];
   // a small world's image is one launch, unless its passes are to be timed one by one
-  const bool one = !timing && image_in_one_launch(W, H);
+  if (one_image < 0) one_image = image_in_one_launch(W, H, stream);
+  const bool one = !timing && one_image == 1;
   Status s = ensure_noise();
   if (!s.ok()) return s;
   CompositeSrc src{};

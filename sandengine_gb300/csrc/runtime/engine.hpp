@@ -133,6 +133,7 @@ struct World {
   float4* d_color = nullptr;
   Status set_light(bool on);
   Status light_frame();  // light pass for the frame just taken (old grid buf[cur ^ 1])
+  int one_image = -1;  // whether the image takes one launch on this stream; -1: not asked yet
   Status ensure_noise();
   Status render_color();  // the current grid's colours into d_color
   // Headless composite of the current grid (colour, its pyramid, the light field when
