@@ -524,7 +524,8 @@ Status World::composite(const float* bg, int bw, int bh) {
   // a small world's image is one launch, unless its passes are to be timed one by one
   if (one_image < 0) one_image = image_in_one_launch(W, H, stream);
   const bool one = !timing && one_image == 1;
-  Status s = ensure_noise();
+  // a caller that holds the colour field's pointer has it follow the images
+  Status s = d_color ? render_color() : ensure_noise();
   if (!s.ok()) return s;
   CompositeSrc src{};
   src.grid = buf[cur];
