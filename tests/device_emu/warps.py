@@ -146,7 +146,7 @@ extern "C" int emu_build_lut() {
 #endif
   g_lut = reinterpret_cast<uint16_t*>(aligned_alloc(256, (bytes + 255) & ~(size_t)255));
   memset(g_lut, 0xee, bytes);
-  gridDim.x = gridDim.y = 1;
+  gridDim.x = gridDim.y = 1, blockIdx.x = blockIdx.y = 0;
   fibers::cta(1, [] { se_build_lut(g_lut); });  // the other builders have no barrier
   for (unsigned w = 0; w < SE_LUT_STATIC_WORDS; ++w) one_thread(w, 0, 1), se_build_static(g_lut);
 #ifdef SE_NIB
