@@ -44,14 +44,17 @@ assert _MOD.size == ctypes.sizeof(SeModification)
 
 def mods_to_c(mods: Sequence[SimModification]):
     arr = (SeModification * max(1, len(mods)))()
+    plain = True
     for i, m in enumerate(mods):
-        try:
-            p = m.position
-            _MOD.pack_into(arr, i * _MOD.size, p[0], p[1], m.mod_shape, m.mod_size, m.mod_matID)
-        except Exception:  # not whole numbers of 32 bits (a float tensor's index raises too): int() and ctypes
-            # truncate, or say what is wrong
-            arr[i].position[0], arr[i].position[1] = int(m.position[0]), int(m.position[1])
-            arr[i].mod_shape, arr[i].mod_size, arr[i].mod_matID = int(m.mod_shape), int(m.mod_size), int(m.mod_matID)
+        if plain:
+            try:
+                p = m.position
+                _MOD.pack_into(arr, i * _MOD.size, p[0], p[1], m.mod_shape, m.mod_size, m.mod_matID)
+                continue
+            except Exception:  # not whole numbers of 32 bits (a float tensor's index raises too): int() and ctypes
+                plain = False  # truncate, or say what is wrong; the rest of the list is likely alike
+        arr[i].position[0], arr[i].position[1] = int(m.position[0]), int(m.position[1])
+        arr[i].mod_shape, arr[i].mod_size, arr[i].mod_matID = int(m.mod_shape), int(m.mod_size), int(m.mod_matID)
     return arr
 
 
