@@ -105,6 +105,7 @@ struct SeNib {
   static constexpr int STRIDE = WPR + (WPR % 4 == 0 ? 2 : 4);
   static constexpr int NG = ((SH + 1) / 2 + LY - 1) / LY, ROWS = 2 * LY * NG + 1;
   static constexpr int TABLE = (STRIDE * ROWS + 3) & ~3;  // the reduced table's first word
+  static constexpr int HIT = TABLE + (SE_NIB_SHARED ? (SE_NIB_ENTRIES + 3) & ~3 : 0);  // that of the edits' bits
 };
 
 // __byte_perm for selectors whose digits are at most 7.
@@ -382,12 +383,12 @@ __device__ __forceinline__ void se_nib_step(uint32_t* sm, bool& look, int ly0, i
   look = 8 * still > seen;
 }
 
-// se_tile_edits (margolus.cuh) on the word-packed array.  A cell is written only by the last
+// se_tile_edits (margolus.cuh) on the word-packed array, for the few mods of most lists.  A cell is written only by the last
 // mod that hits it, so its nibble changes once; the other cells of its word may change at the
 // same time, so the difference is added atomically.
 template <class G, int NT>
-__device__ __forceinline__ void se_nib_edits(uint32_t* sm, int gx0, int gy0, int W, int H, int ya, int yb,
-                                             const SeEditParams* __restrict__ p, int n) {
+__device__ __forceinline__ void se_nib_few_edits(uint32_t* sm, int gx0, int gy0, int W, int H, int ya, int yb,
+                                                 const SeEditParams* __restrict__ p, int n) {
   const int rx0 = gx0 > 0 ? gx0 : 0, rx1 = (gx0 + G::SW < W ? gx0 + G::SW : W) - 1;
   const int ylo = ya > 0 ? ya : 0, yhi = yb < H ? yb : H;
   const int ry0 = gy0 > ylo ? gy0 : ylo, ry1 = (gy0 + G::SH < yhi ? gy0 + G::SH : yhi) - 1;
@@ -411,6 +412,73 @@ __device__ __forceinline__ void se_nib_edits(uint32_t* sm, int gx0, int gy0, int
       if (later || !se_check(i >= 0 && i < G::STRIDE * G::ROWS, 32u)) continue;
       const int d = m.mat - (int)((sm[i] >> sh) & 15u);
       if (d) atomicAdd(reinterpret_cast<int*>(sm) + i, (int)((uint32_t)d << sh));
+    }
+  }
+}
+
+// Longer lists.  Eight words of bits (`hit`, zero before) say which mods' boxes meet the cells
+// that can change: those of the world and of the buffer rows [ya, yb).  After them lie these boxes,
+// clipped to those cells, as array coordinates (x0 | y0 << 16, x1 | y1 << 16).
+template <class G, int NT>
+__device__ __forceinline__ void se_nib_find_edits(uint32_t* hit, int gx0, int gy0, int W, int H, int ya, int yb,
+                                                  const SeEditParams* __restrict__ p, int n) {
+  const int rx0 = se_max(gx0, 0), rx1 = se_min(gx0 + G::SW, W) - 1;
+  const int ry0 = se_max(gy0, se_max(ya, 0)), ry1 = se_min(gy0 + G::SH, se_min(yb, H)) - 1;
+  for (int q = threadIdx.x; q < n; q += NT) {
+    const int4 b = p->boxes[q];
+    const int x0 = se_max(b.x, rx0), y0 = se_max(b.y, ry0), x1 = se_min(b.z, rx1), y1 = se_min(b.w, ry1);
+    if (x0 > x1 || y0 > y1) continue;
+    atomicOr(hit + (q >> 5), 1u << (q & 31));
+    hit[8 + 2 * q] = (uint32_t)(x0 - gx0) | (uint32_t)(y0 - gy0) << 16;
+    hit[9 + 2 * q] = (uint32_t)(x1 - gx0) | (uint32_t)(y1 - gy0) << 16;
+  }
+}
+
+// A cell takes the material of the last mod that hits it unless that is NULL.  A warp takes 32 x 4 cells,
+// a column of four to a lane, finds the mods whose boxes meet them by a vote and goes through these
+// from the last to the first, until each cell has met its last one.  Mod by mod, with a look at all
+// later mods for every cell, the time is that of the fullest tile, and a stroke puts many mods into one
+// (us of a frame on 256 x 256, four materials, waited for, mod by mod / so: 8 circles at random 22.7 / 21.3,
+// 32 58 / 31, 256 690 / 90, 64 circles over each other 636 / 119; columns of eight cells 203).
+template <class G, int NT>
+__device__ __forceinline__ void se_nib_edits(uint32_t* sm, const uint32_t* hit, int gx0, int gy0,
+                                             const SeEditParams* __restrict__ p, int n) {
+  constexpr int WS = NT == 1 ? 1 : 32, R = 4, PX = (G::SW + WS - 1) / WS, PY = (G::SH + R - 1) / R;
+  const int lane = threadIdx.x & (WS - 1);
+  uint32_t any = 0;
+  for (int k = 0; k < (n + 31) >> 5; ++k) any |= hit[k];
+  if (!any) return;
+  for (int i = threadIdx.x / WS; i < PX * PY; i += NT / WS) {
+    const int py = i / PX * R, px = (i - i / PX * PX) * WS, cx = px + lane;
+    uint32_t open = (1u << R) - 1u;  // the lane's cells that no mod has hit yet
+    for (int q0 = (n - 1) / WS * WS; q0 >= 0; q0 -= WS) {
+      if (!(hit[q0 >> 5] >> (WS == 1 ? q0 & 31 : 0))) continue;
+      const int l = q0 + WS - 1 - lane;  // the last mod in the vote's lowest bit
+      bool meets = (hit[l >> 5] >> (l & 31)) & 1u;  // false beyond n
+      if (meets) {
+        const uint32_t lo = hit[8 + 2 * l], hi = hit[9 + 2 * l];
+        meets = (int)(lo & 0xffffu) < px + WS && (int)(hi & 0xffffu) >= px && (int)(lo >> 16) < py + R &&
+                (int)(hi >> 16) >= py;
+      }
+      for (uint32_t m = __ballot_sync(0xffffffffu, meets); m;) {
+        const int q = q0 + WS - __ffs((int)m);
+        m &= m - 1u;
+        const uint32_t lo = hit[8 + 2 * q], hi = hit[9 + 2 * q];
+        if (!open || cx < (int)(lo & 0xffffu) || cx > (int)(hi & 0xffffu)) continue;
+        const SeMod mod = p->mods[q];
+        uint32_t hits = 0;  // all rows at once: the roots in flight together
+#pragma unroll
+        for (int r = 0; r < R; ++r) hits |= se_mod_hits(mod, gx0 + cx, gy0 + py + r) ? 1u << r : 0u;
+        hits &= open & (0xffu << se_max((int)(lo >> 16) - py, 0)) & (0xffu >> se_max(py + 7 - (int)(hi >> 16), 0));
+        open &= ~hits;
+        if (mod.mat == (int)SE_NULL) continue;  // its cells keep the simulated value
+        for (; hits; hits &= hits - 1u) {
+          const int w = (py + __ffs((int)hits) - 1) * G::STRIDE + cx / 8, sh = 4 * (cx & 7);
+          if (!se_check(w >= 0 && w < G::STRIDE * G::ROWS, 32u)) continue;
+          const int d = mod.mat - (int)((sm[w] >> sh) & 15u);
+          if (d) atomicAdd(reinterpret_cast<int*>(sm) + w, (int)((uint32_t)d << sh));
+        }
+      }
     }
   }
 }
@@ -441,6 +509,9 @@ __device__ __forceinline__ void se_nib_run(const uint32_t* __restrict__ src, uin
   const uint32_t umask = NT == 1 ? se_nib_static_mask(lut) : __ldg(gtab + SE_NIB_ENTRIES);
   se_nib_copy_table(tab, gtab, NT);
   const int gx0 = X0 - G::HX, gy0 = Y0 - G::HY;
+  const bool many = nedits > SE_NIB_FEW_EDITS;
+  if (many)
+    for (int i = threadIdx.x; i < 8; i += NT) sm[G::HIT + i] = 0u;
   const bool vec = (W & 3) == 0;
   constexpr int HPR = G::SW / 4;  // half-words (four cells) per row
   uint16_t* sh = reinterpret_cast<uint16_t*>(se_smem);
@@ -494,6 +565,8 @@ __device__ __forceinline__ void se_nib_run(const uint32_t* __restrict__ src, uin
   }
   se_nib_table_ready();
   __syncthreads();
+  if (many)  // read after the first frame's barrier
+    se_nib_find_edits<G, NT>(sm + G::HIT, gx0, gy0, W, H, ya, yb, edits, nedits);
 
   const bool edge = gx0 < 0 || gy0 < 0 || gx0 + G::SW > W || gy0 + G::SH > H;
   bool look = true;
@@ -506,7 +579,10 @@ __device__ __forceinline__ void se_nib_run(const uint32_t* __restrict__ src, uin
       se_nib_step<G, NT, 1>(sm, look, ly0, gx0, gy0, f, W, H, edge, umask, tab, gtab, lut);
     __syncthreads();
     if (s == 0 && nedits > 0) {  // the first frame's edits (the host passes them only then)
-      se_nib_edits<G, NT>(sm, gx0, gy0, W, H, ya, yb, edits, nedits);
+      if (many)
+        se_nib_edits<G, NT>(sm, sm + G::HIT, gx0, gy0, edits, nedits);
+      else
+        se_nib_few_edits<G, NT>(sm, gx0, gy0, W, H, ya, yb, edits, nedits);
       __syncthreads();
     }
   }

@@ -11,6 +11,7 @@
 #include <mutex>
 #include <sstream>
 
+#include "../../../include/sandengine.h"
 #include "kernel_src.inc"  // SE_PRELUDE_SRC, SE_MARGOLUS_SRC, SE_NIBBLE_SRC (generated from csrc/kernels)
 
 namespace se::rt {
@@ -210,12 +211,14 @@ Module::~Module() {
   if (lib) cudaLibraryUnload(lib);
 }
 
-size_t tile_smem_bytes(const TileVariant& t, const LutShape& lut) {
-  if (lut.nib_entries && (t.kmax > 1 || t.small())) {  // SeNib's array (nibble.cuh) and, when small, its reduced table
+size_t tile_smem_bytes(const TileVariant& t, const LutShape& lut, bool edits) {
+  if (lut.nib_entries && (t.kmax > 1 || t.small())) {
+    // SeNib's array (nibble.cuh), the reduced table when small, the bits and boxes of the edits
     const size_t sw16 = (size_t)(t.sw() + 15) / 16, wpr = 2 * ((sw16 + 1) / 2 * 2);
     const size_t stride = wpr + (wpr % 4 == 0 ? 2 : 4);
     const size_t rows = 32 * (((size_t)(t.sh() + 1) / 2 + 15) / 16) + 1;
-    return (((stride * rows + 3) & ~(size_t)3) + (lut.nib_shared ? (lut.nib_entries + 3) & ~3ull : 0)) * 4;
+    return (((stride * rows + 3) & ~(size_t)3) + (lut.nib_shared ? (lut.nib_entries + 3) & ~3ull : 0) +
+            (edits ? 8 + 2 * SE_MAX_MODIFICATIONS : 0)) * 4;
   }
   size_t b = (t.smem_bytes() + 15) & ~(size_t)15;
   // 48-byte header (slack, list counters, uniform-material flags), then the per-step list
@@ -259,7 +262,7 @@ bool Module::load(const std::string& cubin, const LutShape& lut, std::string* er
     if (!t.compiled(lut)) continue;
     for (const std::string& n : {t.name(), t.edit_name(), t.multi_name(), t.serve_name()}) {
       e = cudaFuncSetAttribute((const void*)kernels[n], cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               (int)tile_smem_bytes(t, lut));
+                               (int)tile_smem_bytes(t, lut, n == t.edit_name()));
       if (e != cudaSuccess) {
         *err = std::string("cudaFuncSetAttribute: ") + cudaGetErrorString(e);
         return false;

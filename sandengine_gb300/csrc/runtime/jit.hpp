@@ -54,7 +54,8 @@ const TileVariant* pick_variant(int k, const LutShape& lut, long long cells);
 // Dynamic shared memory of a tile launch: the u8 tile, then the per-step list of chunks to
 // evaluate; or the 4-bit tile and a small reduced table.  The block transition table and its
 // static-key bitset stay in global memory (read through the read-only cache).
-size_t tile_smem_bytes(const TileVariant& t, const LutShape& lut);
+// edits: of the kernel with the edit pass.
+size_t tile_smem_bytes(const TileVariant& t, const LutShape& lut, bool edits = false);
 
 // Full device source: prelude + generated rules + kernel template + instantiations.
 std::string kernel_source(const std::string& generated_rules);

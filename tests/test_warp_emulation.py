@@ -138,7 +138,7 @@ def test_long_edit_lists_with_whole_warps_match_port(se, rulesets, ports):
     rng = np.random.default_rng(14)
     w, h = 231, 117
     for shape in ((56, 30, 1, 128), (48, 48, 8, 128), (112, 112, 8, 256)):
-        for mods in (_mods(rng, w, h, 256), _mods(rng, 40, 40, 256), _mods(rng, w, h, 33) + [(5, 5, 1, 1 << 23, 3)] +
+        for mods in (_mods(rng, w, h, 256), _mods(rng, 30, 30, 4), _mods(rng, 30, 30, 5), _mods(rng, 40, 40, 256), _mods(rng, w, h, 33) + [(5, 5, 1, 1 << 23, 3)] +
                      _mods(rng, w, h, 31)):
             g = _world(rng, w, h, n)
             params, live = _edit_params(n, w, h, mods)
