@@ -637,7 +637,7 @@ SE_API int se_batch_set_steps_per_launch(se_batch* b, int k) {
     const se::rt::TileVariant* v = se::rt::pick_variant(k, b->b->rs->lut_shape(), -1);
     if (!v) return fail(SE_ERR_INVALID_ARGUMENT, "no kernel variant for this many frames per launch");
     b->b->steps_per_launch = k;
-    return ret(b->b->set_variant(v));
+    return ret(b->b->set_variant(v, se::rt::fusion_depth(k)));
   });
 }
 
@@ -674,7 +674,7 @@ SE_API int se_batch_info(const se_batch* b, int* resident_worlds, int* tiled_wor
     if (resident_worlds) *resident_worlds = r;
     if (tiled_worlds) *tiled_worlds = (int)b->b->tiled.size();
     if (cells) *cells = b->b->cells;
-    if (steps_per_launch) *steps_per_launch = b->b->variant ? b->b->variant->kmax : 0;
+    if (steps_per_launch) *steps_per_launch = b->b->variant ? b->b->depth : 0;
     return (int)SE_OK;
   });
 }

@@ -151,7 +151,7 @@ Status Batch::set_resident_limit(size_t bytes) {
   limit_set = true;
   Status s = classify();
   if (!s.ok()) return s;
-  if (variant) return set_variant(variant);  // the tile job list
+  if (variant) return set_variant(variant, depth);  // the tile job list
   return invalidate_graphs();
 }
 
@@ -166,8 +166,9 @@ Status Batch::invalidate_graphs() {
   return Status::Ok();
 }
 
-Status Batch::set_variant(const TileVariant* v) {
+Status Batch::set_variant(const TileVariant* v, int frames) {
   variant = v;
+  depth = frames;
   jobs.clear();
   for (int w : tiled) {
     const WorldDesc& d = desc[(size_t)w];
@@ -214,7 +215,7 @@ Status Batch::set_frame(int i, int32_t f) {
 }
 
 Status Batch::launch_body(int F, cudaStream_t s) {
-  const int k = variant->kmax;
+  const int k = depth;
   const int P = tiled.empty() ? 0 : (F + k - 1) / k;
   const uint16_t* lut = rs->d_lut;
   SE_CUDA(cudaEventRecord(fork, s));
@@ -266,7 +267,7 @@ Status Batch::autotune(int reps, int* best_k) {
     double best_rate = 0;
     for (const TileVariant& v : tile_variants()) {
       if (!v.tuned(rs->lut_shape(), tiled_cells)) continue;
-      Status s = set_variant(&v);
+      Status s = set_variant(&v, v.kmax);
       if (!s.ok()) return s;
       const size_t smem = tile_smem_bytes(v, rs->lut_shape());
       const uint16_t* lut = rs->d_lut;
@@ -290,7 +291,7 @@ Status Batch::autotune(int reps, int* best_k) {
     cudaEventDestroy(a);
     cudaEventDestroy(b);
   }
-  Status s = set_variant(best);
+  Status s = set_variant(best, best->kmax);
   if (!s.ok()) return s;
   if (best_k) *best_k = best->kmax;
   return Status::Ok();
@@ -323,7 +324,7 @@ Status Batch::step(int F) {
     Status s = steps_per_launch > 0 ? Status::Ok() : autotune(2, nullptr);
     if (!s.ok()) return s;
     if (!variant) {
-      s = set_variant(pick_variant(steps_per_launch, rs->lut_shape(), -1));
+      s = set_variant(pick_variant(steps_per_launch, rs->lut_shape(), -1), fusion_depth(steps_per_launch));
       if (!s.ok()) return s;
     }
   }
@@ -342,7 +343,7 @@ Status Batch::step(int F) {
     it = graphs.emplace(F, ex).first;
   }
   SE_CUDA(cudaGraphLaunch(it->second, stream));
-  const int k = variant->kmax;
+  const int k = depth;
   const int P = tiled.empty() ? 0 : (F + k - 1) / k;
   for (auto& d : desc) {
     d.frame += F;

@@ -42,7 +42,8 @@ struct Batch {
   std::vector<Resident> resident;
   std::vector<int> tiled;  // worlds advanced by tile passes
   const TileVariant* variant = nullptr;
-  int steps_per_launch = 0;  // 0: autotune on first use
+  int depth = 0;             // frames a launch of it advances
+  int steps_per_launch = 0;  // as asked for; 0: autotune on first use
   std::vector<TileJob> jobs;
   TileJob* d_jobs = nullptr;
   size_t d_jobs_cap = 0;
@@ -58,7 +59,7 @@ struct Batch {
   Status step(int nframes);
   Status step_plain(int nframes);
   Status autotune(int reps, int* best_k);
-  Status set_variant(const TileVariant* v);
+  Status set_variant(const TileVariant* v, int frames);  // frames per launch, at most v->kmax
   Status invalidate_graphs();
   // Worlds whose whole-world CTA needs at most `bytes` of shared memory stay resident; the
   // others take tile passes (0: none resident).  Rebuilds the classes and the job list.

@@ -70,6 +70,13 @@ const TileVariant* pick_variant(int k, const LutShape& lut, long long cells) {
   return best;
 }
 
+int fusion_depth(int k) {
+  int depth = 0;
+  for (const TileVariant& t : tile_variants())
+    if (t.kmax >= k && (!depth || t.kmax < depth)) depth = t.kmax;
+  return depth;
+}
+
 std::string kernel_source(const std::string& generated_rules) {
   std::ostringstream o;
   o << SE_PRELUDE_SRC << "\n" << generated_rules << "\n" << SE_MARGOLUS_SRC << "\n"

@@ -50,6 +50,9 @@ const std::vector<TileVariant>& tile_variants();
 // The variant for k frames per launch: of those chosen for the rule set's tiles and for worlds of
 // `cells` cells (-1: any) the first with the fewest frames >= k.
 const TileVariant* pick_variant(int k, const LutShape& lut, long long cells);
+// The frames that a launch advances where k are asked for, whichever shape takes it: the fewest
+// >= k of any shape, 0 beyond them all.
+int fusion_depth(int k);
 
 // Dynamic shared memory of a tile launch: the u8 tile, then the per-step list of chunks to
 // evaluate; or the 4-bit tile and a small reduced table.  The block transition table and its

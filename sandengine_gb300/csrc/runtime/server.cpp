@@ -77,6 +77,7 @@ Status Server::set_frames_per_iteration(int k) {
   const TileVariant* v = pick_variant(k, rs->lut_shape(), -1);
   if (!v || k < 1) return {SE_ERR_INVALID_ARGUMENT, "no kernel variant for this many frames per iteration"};
   variant = v;
+  depth = fusion_depth(k);
   small_variant = nullptr;
   if (rs->lut_shape().nib_entries)
     for (const TileVariant& t : tile_variants())
@@ -438,7 +439,7 @@ Status Server::serve_batched(std::unique_lock<std::mutex>& lk) {
     std::stable_sort(pend.begin(), pend.end(),
                      [&](int a, int b) { return requests[(size_t)a].arrival_ms < requests[(size_t)b].arrival_ms; });
   }
-  const int K = variant->kmax;
+  const int K = depth;
   const uint16_t* lut = rs->d_lut;
   size_t next = 0;
   std::deque<int> waiting;  // sessions with queued requests, in order of their turn

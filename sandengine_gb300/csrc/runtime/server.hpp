@@ -66,6 +66,7 @@ struct Server {
   size_t first_pending = 0;   // replay: requests before this index have been served
   size_t last_run_begin = 0;  // first request of the last run
   const TileVariant* variant = nullptr;
+  int depth = 8;  // frames a session advances per iteration, at most
   const TileVariant* small_variant = nullptr;  // for iterations of few cells, as many frames
   cudaStream_t stream = nullptr;
   // pinned staging for per-iteration descriptors, in a ring guarded by events
