@@ -634,10 +634,7 @@ SE_API int se_batch_autotune(se_batch* b, int reps, int* best_k) {
 SE_API int se_batch_set_steps_per_launch(se_batch* b, int k) {
   return guard([&] {
     if (!b || k < 1) return fail(SE_ERR_INVALID_ARGUMENT, "k must be >= 1");
-    const se::rt::TileVariant* v = se::rt::pick_variant(k, b->b->rs->lut_shape(), -1);
-    if (!v) return fail(SE_ERR_INVALID_ARGUMENT, "no kernel variant for this many frames per launch");
-    b->b->steps_per_launch = k;
-    return ret(b->b->set_variant(v, se::rt::fusion_depth(k)));
+    return ret(b->b->set_steps_per_launch(k));
   });
 }
 

@@ -151,6 +151,7 @@ Status Batch::set_resident_limit(size_t bytes) {
   limit_set = true;
   Status s = classify();
   if (!s.ok()) return s;
+  if (steps_per_launch > 0) return set_steps_per_launch(steps_per_launch);
   if (variant) return set_variant(variant, depth);  // the tile job list
   return invalidate_graphs();
 }
@@ -164,6 +165,19 @@ Status Batch::invalidate_graphs() {
   for (auto& kv : graphs) cudaGraphExecDestroy(kv.second);
   graphs.clear();
   return Status::Ok();
+}
+
+long long Batch::tiled_cells() const {
+  long long sum = 0;
+  for (int w : tiled) sum += (long long)desc[(size_t)w].W * desc[(size_t)w].H;
+  return sum;
+}
+
+Status Batch::set_steps_per_launch(int k) {
+  const TileVariant* v = k < 1 ? nullptr : pick_variant(k, rs->lut_shape(), tiled_cells());
+  if (!v) return {SE_ERR_INVALID_ARGUMENT, "no kernel variant for this many frames per launch"};
+  steps_per_launch = k;
+  return set_variant(v, fusion_depth(k));
 }
 
 Status Batch::set_variant(const TileVariant* v, int frames) {
@@ -262,11 +276,10 @@ Status Batch::autotune(int reps, int* best_k) {
     cudaEvent_t a, b;
     SE_CUDA(cudaEventCreate(&a));
     SE_CUDA(cudaEventCreate(&b));
-    long long tiled_cells = 0;
-    for (int w : tiled) tiled_cells += (long long)desc[(size_t)w].W * desc[(size_t)w].H;
+    const long long cells = tiled_cells();
     double best_rate = 0;
     for (const TileVariant& v : tile_variants()) {
-      if (!v.tuned(rs->lut_shape(), tiled_cells)) continue;
+      if (!v.tuned(rs->lut_shape(), cells)) continue;
       Status s = set_variant(&v, v.kmax);
       if (!s.ok()) return s;
       const size_t smem = tile_smem_bytes(v, rs->lut_shape());
@@ -285,12 +298,13 @@ Status Batch::autotune(int reps, int* best_k) {
       SE_CUDA(cudaEventSynchronize(b));
       float ms = 0;
       SE_CUDA(cudaEventElapsedTime(&ms, a, b));
-      const double rate = (double)tiled_cells * v.kmax * reps / (ms > 0 ? ms : 1e-6);
+      const double rate = (double)cells * v.kmax * reps / (ms > 0 ? ms : 1e-6);
       if (rate > best_rate) best_rate = rate, best = &v;
     }
     cudaEventDestroy(a);
     cudaEventDestroy(b);
   }
+  steps_per_launch = 0;
   Status s = set_variant(best, best->kmax);
   if (!s.ok()) return s;
   if (best_k) *best_k = best->kmax;
@@ -321,12 +335,8 @@ Status Batch::step(int F) {
     if (--F == 0) return Status::Ok();
   }
   if (!variant) {
-    Status s = steps_per_launch > 0 ? Status::Ok() : autotune(2, nullptr);
+    Status s = autotune(2, nullptr);
     if (!s.ok()) return s;
-    if (!variant) {
-      s = set_variant(pick_variant(steps_per_launch, rs->lut_shape(), -1), fusion_depth(steps_per_launch));
-      if (!s.ok()) return s;
-    }
   }
   auto it = graphs.find(F);
   if (it == graphs.end()) {

@@ -43,7 +43,7 @@ struct Batch {
   std::vector<int> tiled;  // worlds advanced by tile passes
   const TileVariant* variant = nullptr;
   int depth = 0;             // frames a launch of it advances
-  int steps_per_launch = 0;  // as asked for; 0: autotune on first use
+  int steps_per_launch = 0;  // as asked for; 0: the autotuner's, on first use
   std::vector<TileJob> jobs;
   TileJob* d_jobs = nullptr;
   size_t d_jobs_cap = 0;
@@ -59,6 +59,9 @@ struct Batch {
   Status step(int nframes);
   Status step_plain(int nframes);
   Status autotune(int reps, int* best_k);
+  // k frames per launch, by the shape for what is tiled
+  Status set_steps_per_launch(int k);
+  long long tiled_cells() const;
   Status set_variant(const TileVariant* v, int frames);  // frames per launch, at most v->kmax
   Status invalidate_graphs();
   // Worlds whose whole-world CTA needs at most `bytes` of shared memory stay resident; the

@@ -64,7 +64,7 @@ const TileVariant* pick_variant(int k, const LutShape& lut, long long cells) {
   for (bool ranged : {true, false}) {
     if (best) break;
     for (const TileVariant& t : tile_variants())
-      if (t.kmax >= k && t.fits(lut) && (!ranged || cells < 0 || t.holds(cells)) && (!best || t.kmax < best->kmax))
+      if (t.kmax >= k && t.fits(lut) && (!ranged || t.holds(cells)) && (!best || t.kmax < best->kmax))
         best = &t;
   }
   return best;

@@ -47,8 +47,8 @@ struct TileVariant {
   size_t smem_bytes() const { return (size_t)sw() * (size_t)sh(); }
 };
 const std::vector<TileVariant>& tile_variants();
-// The variant for k frames per launch: of those chosen for the rule set's tiles and for worlds of
-// `cells` cells (-1: any) the first with the fewest frames >= k.
+// The variant for k frames per launch: of those chosen for the rule set's tiles and for `cells` cells
+// (of one world, or of all that a launch advances) the first with the fewest frames >= k.
 const TileVariant* pick_variant(int k, const LutShape& lut, long long cells);
 // The frames that a launch advances where k are asked for, whichever shape takes it: the fewest
 // >= k of any shape, 0 beyond them all.

@@ -69,19 +69,18 @@ Status Server::create(std::shared_ptr<Ruleset> r, long long budget_bytes) {
 Status Server::set_frames_per_iteration(int k) {
   std::lock_guard<std::mutex> g(mu);
   if (live) return {SE_ERR_INVALID_ARGUMENT, "the frames per iteration cannot change while the server runs"};
-  // The first compiled variant with the fewest frames >= k.  For k = 8 on bytes the 128x64 tiles,
-  // which serve sessions of 128-2048 cells a side best (770 G cell-updates/s against 690-734 G
-  // with 256x128, 128x128 or 256x64 tiles: a smaller halo does not make up for the waste on the small
-  // sessions and the coarser work units of an iteration); with two cells a byte 112x112, and
-  // the smaller tiles of as many frames for iterations of few cells (the loop's choice).
-  const TileVariant* v = pick_variant(k, rs->lut_shape(), -1);
-  if (!v || k < 1) return {SE_ERR_INVALID_ARGUMENT, "no kernel variant for this many frames per iteration"};
-  variant = v;
+  // For k = 8 on bytes the 128x64 tiles, which serve sessions of 128-2048 cells a side best (770 G
+  // cell-updates/s against 690-734 G with 256x128, 128x128 or 256x64 tiles: a smaller halo does not
+  // make up for the waste on the small sessions and the coarser work units of an iteration); with two
+  // cells a byte 112x112, and the smallest tiles of as many frames for iterations of few cells (the
+  // loop's choice): for k = 1, 128x64 byte tiles and 56x30.
+  const TileVariant* v = k < 1 ? nullptr : pick_variant(k, rs->lut_shape(), kFewCells + 1);
+  if (!v) return {SE_ERR_INVALID_ARGUMENT, "no kernel variant for this many frames per iteration"};
+  variant = small_variant = v;
   depth = fusion_depth(k);
-  small_variant = nullptr;
   if (rs->lut_shape().nib_entries)
     for (const TileVariant& t : tile_variants())
-      if (!small_variant && t.fits(rs->lut_shape()) && t.kmax == v->kmax && t.tw * t.th < v->tw * v->th)
+      if (t.fits(rs->lut_shape()) && t.kmax == v->kmax && t.tw * t.th < small_variant->tw * small_variant->th)
         small_variant = &t;
   return Status::Ok();
 }
@@ -543,7 +542,7 @@ Status Server::serve_batched(std::unique_lock<std::mutex>& lk) {
     // 112x112 / 48x48: 0.8 million cells 770 / 607, 2.7 million 1180 / 1090, 12.5 million 2878 / 3007).
     long long cells = 0;
     for (int sid : active) cells += (long long)sessions[(size_t)sid].W * sessions[(size_t)sid].H;
-    const TileVariant& v = small_variant && cells <= 1ll << 22 ? *small_variant : *variant;
+    const TileVariant& v = cells <= kFewCells ? *small_variant : *variant;
     int total = 0;
     std::vector<int> ks(active.size());
     for (size_t a = 0; a < active.size(); ++a) {

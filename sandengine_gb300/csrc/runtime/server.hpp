@@ -67,7 +67,8 @@ struct Server {
   size_t last_run_begin = 0;  // first request of the last run
   const TileVariant* variant = nullptr;
   int depth = 8;  // frames a session advances per iteration, at most
-  const TileVariant* small_variant = nullptr;  // for iterations of few cells, as many frames
+  const TileVariant* small_variant = nullptr;  // for iterations of up to kFewCells cells
+  static constexpr long long kFewCells = 1 << 22;
   cudaStream_t stream = nullptr;
   // pinned staging for per-iteration descriptors, in a ring guarded by events
   static constexpr int kRing = 4;
