@@ -31,30 +31,36 @@ std::string TileVariant::edit_name() const {
 // (16-bit offsets in the chunk list).  The arrays of 4-bit tiles take whole warp items of
 // 32 x 32 cells, tile and halo together, so their shapes are 32 n - 2 halo.
 const std::vector<TileVariant>& tile_variants() {
-  constexpr int B = TileVariant::kByte | TileVariant::kTuned, N = TileVariant::kNibble,
-                NT = TileVariant::kNibble | TileVariant::kTuned;
+  constexpr int B = TileVariant::kByte | TileVariant::kByteTuned, N = TileVariant::kNibble,
+                NT = TileVariant::kNibble | TileVariant::kNibbleTuned;
   static const std::vector<TileVariant> v = {
       // one frame of a small world is the latency of a few CTAs: 4-bit tiles of 64 x 32 cells with
       // their halo (us a launch, four materials, 56x30 / 128x64 bytes: 64^2 to 512^2 4.2 / 8.2, 1024^2
       // 6.2 / 8.3, 2048^2 8.3 / 11.4; twelve 4.1 / 7.6, 6.2 / 8.3, 10.3 / 12.3)
       {56, 30, 1, 128, NT, 0, 1 << 22},
-      {128, 64, 1, 256, B | N},  {256, 32, 1, 256, B | N}, {128, 32, 1, 256, B | N}, {128, 64, 2, 256, B},
-      {128, 64, 4, 256, B},      {128, 64, 8, 256, B},     {128, 128, 8, 256, B},    {128, 128, 16, 256, B},
-      {256, 64, 4, 256, B},      {64, 64, 4, 256, B},      {256, 128, 8, 512, B},    {192, 128, 8, 256, B},
+      {128, 64, 1, 256, B | NT}, {256, 32, 1, 256, B | NT}, {128, 32, 1, 256, B | NT}, {128, 64, 2, 256, B},
+      {128, 64, 4, 256, B},      {128, 64, 8, 256, B},      {128, 128, 8, 256, B},
+      {256, 64, 4, 256, B},      {64, 64, 4, 256, B},       {256, 128, 8, 512, B},     {192, 128, 8, 256, B},
       {256, 128, 4, 512, B},     {256, 64, 8, 256, B},
       // 32x32 and 48x48 for the latency of small worlds, the large ones for the rate of large ones,
       // 96x96 between (us a frame, four materials, 32x32_k16 / 48x48_k8 / 96x96_k16 / 112x112_k8 /
       // 240x176_k8: 256^2 0.66 / 1.07 / 1.18 / 1.60 / 3.64, 1024^2 1.31 / 1.34 / 1.18 / 1.61 / 3.41, 4096^2 14.4
       // / 8.7 / 7.2 / 7.0 / 6.5; three 4096^2 worlds at once, 60 frames of one: 852 / 489 / 387 / 362 / 313 us).
-      // The autotuner tries those whose range holds the world; 120x120 serves callers that ask for
-      // 2 to 4 frames a launch.
-      {120, 120, 4, 128, N},
+      // The autotuner tries those whose range holds the world; 120x120 is for callers that ask for 2 to
+      // 4 frames a launch on large worlds, where the smaller halo pays for its few threads (us of 2 and 4
+      // frames, twelve, 120x120_k4 / 240x176_k8 / 112x112_k8: 8192^2 119 154 / 135 184 / 130 177; 3001x2003 33 38 /
+      // 36 44 / 31 39; 1000x700 25 32 / 30 39 / 20 24).
+      {120, 120, 4, 128, N, 1 << 23},
       {112, 112, 8, 256, NT, 1 << 18},
       {48, 48, 8, 128, NT, 0, 1 << 23},
       {240, 176, 8, 256, NT, 1 << 22},
       {240, 240, 8, 256, NT, 1 << 23},
       {96, 96, 16, 256, NT, 0, 1 << 22},
       {32, 32, 16, 128, NT, 0, 1 << 20},
+      // on 4-bit cells for callers that ask for 16 frames a launch on large worlds (us of 48 frames, four
+      // materials, 128x128_k16 / 96x96_k16: 8192^2 1171 / 1262, 4096^2 352 / 363, 2500^2 182 / 163; twelve
+      // 1679 / 1892, 513 / 554, 259 / 277)
+      {128, 128, 16, 256, B | N, 1 << 24},
   };
   return v;
 }
@@ -64,7 +70,7 @@ const TileVariant* pick_variant(int k, const LutShape& lut, long long cells) {
   for (bool ranged : {true, false}) {
     if (best) break;
     for (const TileVariant& t : tile_variants())
-      if (t.kmax >= k && t.fits(lut) && (!ranged || t.holds(cells)) && (!best || t.kmax < best->kmax))
+      if (t.kmax >= k && t.fits(lut) && (!ranged || t.holds(lut, cells)) && (!best || t.kmax < best->kmax))
         best = &t;
   }
   return best;

@@ -24,17 +24,19 @@ struct LutShape {
 // A tile-kernel instantiation: TW x TH output cells, up to KMAX frames per launch.
 struct TileVariant {
   int tw, th, kmax, nt;
-  enum { kByte = 1, kNibble = 2, kTuned = 4 };
-  int use;  // the kinds of tile it is chosen for, and whether by the autotuner (set_tile may ask for any)
-  long long min_cells = 0, max_cells = 1ll << 62;
+  enum { kByte = 1, kNibble = 2, kByteTuned = 4, kNibbleTuned = 8 };
+  int use;  // the kinds of tile it is chosen for, and tried for by the autotuner (set_tile may ask for any)
+  long long min_cells = 0, max_cells = 1ll << 62;  // as a 4-bit tile, for worlds of so many cells
   // Whether the rule set's module holds it: shapes for 4-bit tiles only where there are such.
   bool compiled(const LutShape& lut) const { return (use & kByte) || lut.nib_entries; }
   bool fits(const LutShape& lut) const { return use & (lut.nib_entries ? kNibble : kByte); }
   // Whether the autotuner tries it on `cells` cells (of one world, or of a batch's tiled worlds).
   bool tuned(const LutShape& lut, long long cells) const {
-    return fits(lut) && (use & kTuned) && holds(cells);
+    return (use & (lut.nib_entries ? kNibbleTuned : kByteTuned)) && holds(lut, cells);
   }
-  bool holds(long long cells) const { return cells >= min_cells && cells <= max_cells; }
+  bool holds(const LutShape& lut, long long cells) const {
+    return !lut.nib_entries || (cells >= min_cells && cells <= max_cells);
+  }
   bool small() const { return tw * th <= 2048; }  // one-frame tiles on 4-bit cells (se_tile_run)
   std::string name() const;        // single-world kernel
   std::string edit_name() const;   // single-world kernel with the first frame's edit pass

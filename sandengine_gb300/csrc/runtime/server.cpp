@@ -72,16 +72,17 @@ Status Server::set_frames_per_iteration(int k) {
   // For k = 8 on bytes the 128x64 tiles, which serve sessions of 128-2048 cells a side best (770 G
   // cell-updates/s against 690-734 G with 256x128, 128x128 or 256x64 tiles: a smaller halo does not
   // make up for the waste on the small sessions and the coarser work units of an iteration); with two
-  // cells a byte 112x112, and the smallest tiles of as many frames for iterations of few cells (the
-  // loop's choice): for k = 1, 128x64 byte tiles and 56x30.
-  const TileVariant* v = k < 1 ? nullptr : pick_variant(k, rs->lut_shape(), kFewCells + 1);
+  // cells a byte 112x112, and the smallest tiles of as many frames, 48x48, for iterations of few cells (the
+  // loop's choice).
+  const TileVariant* v = k < 1 ? nullptr : pick_variant(k, rs->lut_shape(), 1 << 23);
   if (!v) return {SE_ERR_INVALID_ARGUMENT, "no kernel variant for this many frames per iteration"};
-  variant = small_variant = v;
-  depth = fusion_depth(k);
+  variant = v;
+  small_variant = pick_variant(k, rs->lut_shape(), 1 << 17);
   if (rs->lut_shape().nib_entries)
     for (const TileVariant& t : tile_variants())
-      if (t.fits(rs->lut_shape()) && t.kmax == v->kmax && t.tw * t.th < small_variant->tw * small_variant->th)
+      if (t.fits(rs->lut_shape()) && t.kmax == small_variant->kmax && t.tw * t.th < small_variant->tw * small_variant->th)
         small_variant = &t;
+  depth = fusion_depth(k);
   return Status::Ok();
 }
 

@@ -17,7 +17,7 @@ from tests.device_emu.emu import HERE, OUT
 
 # (tile width, tile height, frames, threads) of the 4-bit tile shapes, and three byte shapes
 SHAPES = [(56, 30, 1, 128), (120, 120, 4, 128), (112, 112, 8, 256), (48, 48, 8, 128), (240, 176, 8, 256),
-          (240, 240, 8, 256), (96, 96, 16, 256), (32, 32, 16, 128)]
+          (240, 240, 8, 256), (96, 96, 16, 256), (32, 32, 16, 128), (128, 128, 16, 256)]
 BYTE_SHAPES = [(128, 64, 1, 256), (128, 64, 8, 256), (64, 64, 4, 256)]
 
 PRELUDE = r'''
