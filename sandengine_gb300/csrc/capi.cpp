@@ -372,6 +372,7 @@ SE_API int se_world_set_tile(se_world* w, int tile_w, int tile_h, int k) {
           W.single = &t;
         } else {
           W.fused = &t;
+          W.tile_asked = true;
           W.steps_per_launch = 0;
         }
         return (int)SE_OK;

@@ -224,6 +224,7 @@ Status World::autotune(int reps, int* best_k) {
   cudaEventDestroy(b);
   fused = vm;
   single = v1;
+  tile_asked = false;
   if (best_k) *best_k = vm ? vm->kmax : 1;
   return Status::Ok();
 }
@@ -393,6 +394,9 @@ Status World::step(int nframes, const se_modification* mods, int nmods) {
     vmulti = fused ? fused : vone;
   }
   const int kdef = steps_per_launch > 0 ? steps_per_launch : vmulti->kmax;
+  // a call's last frames, fewer than its launches take: a shape of few frames where one is meant for
+  // the world (tile_variants), unless the caller has chosen the tile
+  const bool few = steps_per_launch == 0 && !tile_asked && rs->lut_shape().nib_entries > 0;
   if (light[0]) {  // one frame at a time, each followed by the light pass
     for (int i = 0; i < nframes; ++i) {
       const int f = frame + 1 + i;
@@ -423,6 +427,10 @@ Status World::step(int nframes, const se_modification* mods, int nmods) {
     }
     const int k = std::min(kdef, nframes - i);
     const TileVariant* v = k == 1 ? vone : vmulti;
+    if (few && k > 1 && k < kdef) {
+      const TileVariant* t = pick_variant(k, rs->lut_shape(), (long long)W * H);
+      if (t->kmax < 8) v = t;
+    }
     if (i == 0 && nlive > 0) {  // the edit pass runs inside the launch, after its first frame
       fill_edit_params(*rs, W, ya, H, mods, nlive, &edit_params);
       Status s = launch_tiles(f, k, v, true, &edit_params, nlive);

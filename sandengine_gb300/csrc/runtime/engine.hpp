@@ -91,6 +91,7 @@ struct World {
   int steps_per_launch = 0;  // 0: chosen by the autotuner on the first multi-frame step
   const TileVariant* fused = nullptr;   // variant for multi-frame launches
   const TileVariant* single = nullptr;  // variant for one-frame launches (edit frames)
+  bool tile_asked = false;              // fused is the caller's choice, not the autotuner's
   ~World();
   Status create(std::shared_ptr<Ruleset> r, int w, int h);
   // The band [row0, row0 + rows) of a w x world_h world with `halo` rows either side.

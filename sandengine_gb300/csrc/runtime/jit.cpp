@@ -46,8 +46,8 @@ const std::vector<TileVariant>& tile_variants() {
       // 96x96 between (us a frame, four materials, 32x32_k16 / 48x48_k8 / 96x96_k16 / 112x112_k8 /
       // 240x176_k8: 256^2 0.66 / 1.07 / 1.18 / 1.60 / 3.64, 1024^2 1.31 / 1.34 / 1.18 / 1.61 / 3.41, 4096^2 14.4
       // / 8.7 / 7.2 / 7.0 / 6.5; three 4096^2 worlds at once, 60 frames of one: 852 / 489 / 387 / 362 / 313 us).
-      // The autotuner tries those whose range holds the world; 120x120 is for callers that ask for 2 to
-      // 4 frames a launch on large worlds, where the smaller halo pays for its few threads (us of 2 and 4
+      // The autotuner tries those whose range holds the world; 120x120 is for 2 to 4 frames of large worlds,
+      // asked for or left at the end of a call, where the smaller halo pays for its few threads (us of 2 and 4
       // frames, twelve, 120x120_k4 / 240x176_k8 / 112x112_k8: 8192^2 119 154 / 135 184 / 130 177; 3001x2003 33 38 /
       // 36 44 / 31 39; 1000x700 25 32 / 30 39 / 20 24).
       {120, 120, 4, 128, N, 1 << 23},

@@ -27,6 +27,23 @@ def _world(se, rulesets, ports, size):
     return sim, run
 
 
+@pytest.mark.parametrize("size, big", [((4096, 2048), True), ((4095, 2048), False)])
+def test_last_frames_of_a_call(se, rulesets, ports, size, big):
+    sim, run = _world(se, rulesets, ports, size)
+    sim.autotune()
+    full = "se_tile_%dx%d_k%d" % sim.tile()
+    few = "se_tile_120x120_k4" if big else full
+    for frames in (2, 4, 3):
+        assert run(frames) == [few]
+    assert run(sim.tile()[2] + 3) == sorted({full, few})
+    assert run(3, edits=True) == [few.replace("tile", "tile_edit")]
+    assert run(5) == [full]
+    sim.set_tile(48, 48, 8)  # the caller's choice holds for every launch
+    assert run(3) == ["se_tile_48x48_k8"]
+    sim.autotune()
+    assert "se_tile_48x48_k8" not in run(3) or not big
+
+
 @pytest.mark.parametrize("size, shapes", [
     ((64, 64), {2: "48x48_k8", 3: "48x48_k8", 4: "48x48_k8", 8: "48x48_k8", 16: "96x96_k16"}),
     ((1001, 777), {2: "112x112_k8", 4: "112x112_k8", 8: "112x112_k8", 16: "96x96_k16"}),
