@@ -138,7 +138,7 @@ int se_world_set_light_field(se_world* w, const float* rgba, size_t n_floats);
 int se_world_render_color(se_world* w, float* rgba, size_t n_floats);
 /* The same into the world's own device buffer, ordered on the world's stream (no
  * synchronization); *rgba stays valid until se_world_destroy.  From the first
- * se_world_render_color* call on, every se_world_composite* call renders the buffer anew. */
+ * such call on, every se_world_composite* call renders the buffer anew. */
 int se_world_render_color_device(se_world* w, float** rgba);
 
 /* Headless composite of the current grid (shaders/fragment140.glsl:70-100, drawn by

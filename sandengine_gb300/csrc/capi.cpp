@@ -285,6 +285,7 @@ SE_API int se_world_render_color_device(se_world* w, float** rgba) {
     if (!w || !rgba) return fail(SE_ERR_INVALID_ARGUMENT, "null argument");
     se::rt::Status s = w->w->render_color();
     if (!s.ok()) return ret(s);
+    w->w->color_shared = true;
     *rgba = reinterpret_cast<float*>(w->w->d_color);
     return (int)SE_OK;
   });

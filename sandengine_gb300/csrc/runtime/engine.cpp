@@ -533,7 +533,7 @@ Status World::composite(const float* bg, int bw, int bh) {
   if (one_image < 0) one_image = image_in_one_launch(W, H, stream);
   const bool one = !timing && one_image == 1;
   // a caller that holds the colour field's pointer has it follow the images
-  Status s = d_color ? render_color() : ensure_noise();
+  Status s = color_shared ? render_color() : ensure_noise();
   if (!s.ok()) return s;
   CompositeSrc src{};
   src.grid = buf[cur];

@@ -132,6 +132,7 @@ struct World {
   int lcur = 0;
   float* d_noise = nullptr;
   float4* d_color = nullptr;
+  bool color_shared = false;  // a caller holds its pointer
   Status set_light(bool on);
   Status light_frame();  // light pass for the frame just taken (old grid buf[cur ^ 1])
   int one_image = -1;  // whether the image takes one launch on this stream; -1: not asked yet
