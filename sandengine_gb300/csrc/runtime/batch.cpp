@@ -180,21 +180,37 @@ Status Batch::set_steps_per_launch(int k) {
   return set_variant(v, fusion_depth(k));
 }
 
+size_t Batch::count_jobs(const TileVariant& v) const {
+  size_t sum = 0;
+  for (int w : tiled) {
+    const WorldDesc& d = desc[(size_t)w];
+    sum += (size_t)((d.W + v.tw - 1) / v.tw) * (size_t)((d.H + v.th - 1) / v.th);
+  }
+  return sum;
+}
+
+Status Batch::reserve_jobs(size_t count) {
+  if (count <= d_jobs_cap) return Status::Ok();
+  if (d_jobs) cudaFree(d_jobs);
+  d_jobs = nullptr;
+  d_jobs_cap = 0;
+  SE_CUDA(cudaMalloc(&d_jobs, count * sizeof(TileJob)));
+  d_jobs_cap = count;
+  return Status::Ok();
+}
+
 Status Batch::set_variant(const TileVariant* v, int frames) {
   variant = v;
   depth = frames;
   jobs.clear();
+  jobs.reserve(count_jobs(*v));
   for (int w : tiled) {
     const WorldDesc& d = desc[(size_t)w];
     for (int y = 0; y < d.H; y += v->th)
       for (int x = 0; x < d.W; x += v->tw) jobs.push_back(TileJob{w, x, y, 0});
   }
-  if (jobs.size() > d_jobs_cap) {
-    if (d_jobs) cudaFree(d_jobs);
-    d_jobs = nullptr;
-    SE_CUDA(cudaMalloc(&d_jobs, jobs.size() * sizeof(TileJob)));
-    d_jobs_cap = jobs.size();
-  }
+  Status s = reserve_jobs(jobs.size());
+  if (!s.ok()) return s;
   if (!jobs.empty())
     SE_CUDA(cudaMemcpyAsync(d_jobs, jobs.data(), jobs.size() * sizeof(TileJob), cudaMemcpyHostToDevice, stream));
   SE_CUDA(cudaStreamSynchronize(stream));
@@ -277,9 +293,20 @@ Status Batch::autotune(int reps, int* best_k) {
     SE_CUDA(cudaEventCreate(&a));
     SE_CUDA(cudaEventCreate(&b));
     const long long cells = tiled_cells();
-    double best_rate = 0;
+    // 4-bit shapes of one frame never win here (they leave a frame's launch to each frame), and trials are
+    // most of a small batch's first step, so they are left out, and the job list grows once.
+    std::vector<const TileVariant*> shapes;
+    size_t most = 0;
     for (const TileVariant& v : tile_variants()) {
-      if (!v.tuned(rs->lut_shape(), cells)) continue;
+      if (!v.tuned(rs->lut_shape(), cells) || (rs->lut_shape().nib_entries && v.kmax == 1)) continue;
+      shapes.push_back(&v);
+      most = std::max(most, count_jobs(v));
+    }
+    Status reserved = reserve_jobs(most);
+    if (!reserved.ok()) return reserved;
+    double best_rate = 0;
+    for (const TileVariant* shape : shapes) {
+      const TileVariant& v = *shape;
       Status s = set_variant(&v, v.kmax);
       if (!s.ok()) return s;
       const size_t smem = tile_smem_bytes(v, rs->lut_shape());

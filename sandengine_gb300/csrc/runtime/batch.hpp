@@ -62,6 +62,8 @@ struct Batch {
   // k frames per launch, by the shape for what is tiled
   Status set_steps_per_launch(int k);
   long long tiled_cells() const;
+  size_t count_jobs(const TileVariant& v) const;
+  Status reserve_jobs(size_t count);
   Status set_variant(const TileVariant* v, int frames);  // frames per launch, at most v->kmax
   Status invalidate_graphs();
   // Worlds whose whole-world CTA needs at most `bytes` of shared memory stay resident; the
