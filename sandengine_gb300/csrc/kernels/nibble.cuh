@@ -102,7 +102,8 @@ struct SeNib {
   static constexpr int LX = 2, LY = 16;  // a warp takes LX chunks of LY block rows: 32 x 32 cells
   static constexpr int SW = ((TW + 2 * HX + 15) / 16) * 16, SH = TH + 2 * HY;
   static constexpr int CPR = (SW / 16 + LX - 1) / LX * LX, WPR = 2 * CPR;  // chunks, words a row
-  static constexpr int STRIDE = WPR + (WPR % 4 == 0 ? 2 : 4);
+  static constexpr int STRIDE = WPR + 2;
+  static_assert(WPR % 4 == 0, "a row's chunks come in pairs");
   static constexpr int NG = ((SH + 1) / 2 + LY - 1) / LY, ROWS = 2 * LY * NG + 1;
   static constexpr int TABLE = (STRIDE * ROWS + 3) & ~3;  // the reduced table's first word
   static constexpr int HIT = TABLE + (SE_NIB_SHARED ? (SE_NIB_ENTRIES + 3) & ~3 : 0);  // that of the edits' bits

@@ -102,6 +102,8 @@ std::string kernel_source(const std::string& generated_rules) {
          " int nedits) {\n"
       << "  se_tile_impl<" << t.tw << ", " << t.th << ", " << t.kmax << ", " << t.nt
       << ">(src, dst, W, H, f0, k, lut, ya, yb, &edits, nedits);\n}\n";
+    // batches and servers take the shapes chosen for the rule set's tiles; a world any, by set_tile
+    if (!(t.use & TileVariant::kNibble)) o << "#ifndef SE_NIB\n";
     o << "extern \"C\" __global__ void " << bounds << t.multi_name()
       << "(const SeWorldDesc* __restrict__ worlds, const SeTileJob* __restrict__ jobs, int pass,"
          " int frames_done, int k, const uint16_t* __restrict__ lut) {\n"
@@ -112,7 +114,7 @@ std::string kernel_source(const std::string& generated_rules) {
          " const uint16_t* __restrict__ lut) {\n"
       << "  se_stile_impl<" << t.tw << ", " << t.th << ", " << t.kmax << ", " << t.nt
       << ">(descs, prefix, nactive, lut);\n}\n";
-    if (!(t.use & TileVariant::kByte)) o << "#endif\n";
+    if (!(t.use & TileVariant::kByte) || !(t.use & TileVariant::kNibble)) o << "#endif\n";
   }
   return o.str();
 }
@@ -228,7 +230,7 @@ size_t tile_smem_bytes(const TileVariant& t, const LutShape& lut, bool edits) {
   if (lut.nib_entries && (t.kmax > 1 || t.small())) {
     // SeNib's array (nibble.cuh), the reduced table when small, the bits and boxes of the edits
     const size_t sw16 = (size_t)(t.sw() + 15) / 16, wpr = 2 * ((sw16 + 1) / 2 * 2);
-    const size_t stride = wpr + (wpr % 4 == 0 ? 2 : 4);
+    const size_t stride = wpr + 2;
     const size_t rows = 32 * (((size_t)(t.sh() + 1) / 2 + 15) / 16) + 1;
     return (((stride * rows + 3) & ~(size_t)3) + (lut.nib_shared ? (lut.nib_entries + 3) & ~3ull : 0) +
             (edits ? 8 + 2 * SE_MAX_MODIFICATIONS : 0)) * 4;
@@ -257,6 +259,7 @@ bool Module::load(const std::string& cubin, const LutShape& lut, std::string* er
     if (!t.compiled(lut)) continue;
     names.push_back(t.name());
     names.push_back(t.edit_name());
+    if (!t.fits(lut)) continue;
     names.push_back(t.multi_name());
     names.push_back(t.serve_name());
   }
@@ -274,6 +277,7 @@ bool Module::load(const std::string& cubin, const LutShape& lut, std::string* er
     tiles.push_back(t.compiled(lut) ? kernels[t.edit_name()] : nullptr);
     if (!t.compiled(lut)) continue;
     for (const std::string& n : {t.name(), t.edit_name(), t.multi_name(), t.serve_name()}) {
+      if (!kernels.count(n)) continue;
       e = cudaFuncSetAttribute((const void*)kernels[n], cudaFuncAttributeMaxDynamicSharedMemorySize,
                                (int)tile_smem_bytes(t, lut, n == t.edit_name()));
       if (e != cudaSuccess) {
