@@ -731,9 +731,6 @@ __device__ __forceinline__ uint4 se_load_quad(const uint32_t* __restrict__ src, 
 #define SE_NIB_SHARED (SE_NMAT <= 8)
 #define SE_NIB_ENTRIES (SE_NIB_SHARED ? SE_NMAT * SE_NMAT * SE_NMAT * SE_NMAT : 65536)
 #define SE_NIB_BOUNDS ((SE_NIB_ENTRIES + 4) & ~3)  // the bound table's first word
-// Edit lists up to this long are applied mod by mod (se_nib_few_edits; us of a frame on 256 x 256, four
-// materials, waited for, so / the lists' way: 1 circle 14.9 / 16.7, 2 15.5 / 17.2, 4 23.4 / 21.8).
-#define SE_NIB_FEW_EDITS 4
 // Launch bounds of the multi-frame tile kernels: up to 64 registers, for eight lookups and eight hashes of
 // a lane in flight (32 warps an SM; 40 or 48 at 48 or 40 registers ran 1% and 5% slower).
 #define SE_TILE_BOUNDS(NT) __launch_bounds__(NT, 1024 / NT)

@@ -241,7 +241,7 @@ Status launch_tile_kernel(const Ruleset& rs, const TileVariant& v, const uint32_
   void* args[] = {(void*)&src, (void*)&dst, &W, &H, &f0, &k, (void*)&lut, &ya, &yb, (void*)edits, &nedits};
   dim3 grid((unsigned)((W + v.tw - 1) / v.tw), (unsigned)((yb - ya + v.th - 1) / v.th));
   SE_CUDA(cudaLaunchKernel((const void*)kern, grid, dim3((unsigned)v.nt), args,
-                           tile_smem_bytes(v, rs.lut_shape(), edits != nullptr), stream));
+                           tile_smem_bytes(v, rs.lut_shape(), edits ? nedits : 0), stream));
   return Status::Ok();
 }
 

@@ -85,6 +85,7 @@ int fusion_depth(int k) {
 
 std::string kernel_source(const std::string& generated_rules) {
   std::ostringstream o;
+  o << "#define SE_NIB_FEW_EDITS " << kFewEdits << "\n";
   o << SE_PRELUDE_SRC << "\n" << generated_rules << "\n" << SE_MARGOLUS_SRC << "\n"
     << SE_NIBBLE_SRC << "\n";
   for (const TileVariant& t : tile_variants()) {
@@ -226,14 +227,14 @@ Module::~Module() {
   if (lib) cudaLibraryUnload(lib);
 }
 
-size_t tile_smem_bytes(const TileVariant& t, const LutShape& lut, bool edits) {
+size_t tile_smem_bytes(const TileVariant& t, const LutShape& lut, int nedits) {
   if (lut.nib_entries && (t.kmax > 1 || t.small())) {
     // SeNib's array (nibble.cuh), the reduced table when small, the bits and boxes of the edits
     const size_t sw16 = (size_t)(t.sw() + 15) / 16, wpr = 2 * ((sw16 + 1) / 2 * 2);
     const size_t stride = wpr + 2;
     const size_t rows = 32 * (((size_t)(t.sh() + 1) / 2 + 15) / 16) + 1;
     return (((stride * rows + 3) & ~(size_t)3) + (lut.nib_shared ? (lut.nib_entries + 3) & ~3ull : 0) +
-            (edits ? 8 + 2 * SE_MAX_MODIFICATIONS : 0)) * 4;
+            (nedits > kFewEdits ? 8 + 2 * SE_MAX_MODIFICATIONS : 0)) * 4;
   }
   size_t b = (t.smem_bytes() + 15) & ~(size_t)15;
   // 48-byte header (slack, list counters, uniform-material flags), then the per-step list
@@ -279,7 +280,7 @@ bool Module::load(const std::string& cubin, const LutShape& lut, std::string* er
     for (const std::string& n : {t.name(), t.edit_name(), t.multi_name(), t.serve_name()}) {
       if (!kernels.count(n)) continue;
       e = cudaFuncSetAttribute((const void*)kernels[n], cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               (int)tile_smem_bytes(t, lut, n == t.edit_name()));
+                               (int)tile_smem_bytes(t, lut, n == t.edit_name() ? SE_MAX_MODIFICATIONS : 0));
       if (e != cudaSuccess) {
         *err = std::string("cudaFuncSetAttribute: ") + cudaGetErrorString(e);
         return false;

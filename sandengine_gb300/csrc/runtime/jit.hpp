@@ -56,11 +56,16 @@ const TileVariant* pick_variant(int k, const LutShape& lut, long long cells);
 // >= k of any shape, 0 beyond them all.
 int fusion_depth(int k);
 
+// Edit lists up to this long are applied mod by mod in 4-bit tiles (se_nib_few_edits; us of a frame on
+// 256 x 256, four materials, waited for, so / the longer lists' way: 1 circle 14.9 / 16.7, 2 15.5 / 17.2, 4
+// 23.4 / 21.8).
+constexpr int kFewEdits = 4;
 // Dynamic shared memory of a tile launch: the u8 tile, then the per-step list of chunks to
 // evaluate; or the 4-bit tile and a small reduced table.  The block transition table and its
 // static-key bitset stay in global memory (read through the read-only cache).
-// edits: of the kernel with the edit pass.
-size_t tile_smem_bytes(const TileVariant& t, const LutShape& lut, bool edits = false);
+// nedits: the mods of an edit launch; the bits and boxes of a long list take 2 KB, which shorter ones leave
+// to L1 (frame, light and image of 1920 x 1080, twelve materials, two mods: 51.2 us with them, 50.8 without).
+size_t tile_smem_bytes(const TileVariant& t, const LutShape& lut, int nedits = 0);
 
 // Full device source: prelude + generated rules + kernel template + instantiations.
 std::string kernel_source(const std::string& generated_rules);
