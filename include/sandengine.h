@@ -179,7 +179,8 @@ int se_world_get_stream(se_world* w, void** cuda_stream);
 int se_world_set_steps_per_launch(se_world* w, int k);
 /* Times every compiled tile shape and fusion depth on this world (`reps` launches each,
  * reading the current grid into the spare buffer, so the world's state is unchanged) and
- * keeps the fastest; *best_k gets the chosen frames per launch.  (No counterpart in the
+ * keeps the best: the fastest, with 4-bit tiles the fastest after a weight on halo cells, which
+ * other worlds on the chip would pay for; *best_k gets the chosen frames per launch.  (No counterpart in the
  * reference, which dispatches one frame at a time.) */
 int se_world_autotune(se_world* w, int reps, int* best_k);
 /* Chooses the compiled tile variant for multi-frame launches (k >= 2) or for one-frame
@@ -292,6 +293,8 @@ int se_batch_step_plain(se_batch* b, int nframes);
 /* Times every tile shape / fusion depth on the tiled worlds (state unchanged) and keeps
  * the fastest; *best_k = frames per tile pass. */
 int se_batch_autotune(se_batch* b, int reps, int* best_k);
+/* Frames per tile pass: the least compiled depth (1, 2, 4, 8, 16) that holds k, on the tile shape
+ * for the cells that are tiled. */
 int se_batch_set_steps_per_launch(se_batch* b, int k);
 /* Worlds whose whole-world CTA needs at most `bytes` of shared memory are advanced in
  * shared memory for all frames of a launch group; the others by tile passes (0: all by tile
@@ -327,7 +330,8 @@ typedef struct se_server_stats {
  * first, and restored when a request needs them. */
 int se_server_create(se_ruleset* rs, long long budget_bytes, se_server** out);
 void se_server_destroy(se_server* s);
-/* Frames a session may advance per batched iteration (a compiled fusion depth). */
+/* Frames a session may advance per batched iteration: the least compiled depth (1, 2, 4, 8, 16)
+ * that holds k. */
 int se_server_set_frames_per_iteration(se_server* s, int k);
 /* A session with an initial grid (NULL = all EMPTY) and frame counter. */
 int se_server_open_session(se_server* s, int width, int height, const uint32_t* cells, int32_t frame,

@@ -634,7 +634,8 @@ __device__ __forceinline__ void se_nib_world_step(uint32_t* sm, int stride, int 
 
 // se_resident's body on a word-packed array: the whole world with a WALL border of 4 columns on
 // the left, at least one on the right, and one row above and below; two words of padding per
-// row.  A world takes half a byte a cell, so worlds of up to about 450,000 cells fit a CTA.  Bound as
+// row (the stride is 0 mod 4 words where cpr is odd: some of its 8-byte accesses meet in a bank, unlike a
+// tile's).  A world takes half a byte a cell, so worlds of up to about 450,000 cells fit a CTA.  Bound as
 // the tiles are (4096 worlds, 100 frames, on byte arrays / so: 28.5 / 23.5 ms).
 __device__ __forceinline__ void se_nib_resident(const SeWorldDesc& w, int frames, int out_flip,
                                                 const uint16_t* __restrict__ lut) {

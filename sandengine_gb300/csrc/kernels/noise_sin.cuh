@@ -72,7 +72,7 @@ __device__ __forceinline__ uint64_t mulhi_short(uint64_t a, uint64_t b) {
 // Terms 7 to 3 take 32-bit steps, scaled to 2^59 .. 2^36; each is off by under 2 units, so
 // the sum from v^3 on by 2 * 2^-36 * 2^-6 = 2^-41; the omitted terms are below 2^-49, the
 // 64-bit steps off by some units of 2^-62.  The bound is 2^-40 (2^-40 u + 2^-56 with the factor u).
-// Compared on the CPU for every binary32 number of the range: no bit differs.
+// tests/test_noise_sine.py compares every binary32 number of the range on the CPU.
 __device__ __forceinline__ float se_sin_fast(float xf) {
   const uint32_t bits = __float_as_uint(xf);
   const uint32_t ex = (bits >> 23) & 255u;

@@ -97,7 +97,7 @@ Status Batch::classify() {
   const size_t maxsm = rs->module->max_dyn_smem;
   const LutShape lut = rs->lut_shape();
   // Size classes for whole-world CTAs: occupancy is set by the largest world of a class.  A
-  // 4-bit world has one chunk of 16 x 2 cells per 16 bytes: two to eight chunks a lane.
+  // 4-bit world has one chunk of 16 x 2 cells per 16 bytes: up to 4, 4, 6 and about 14 chunks a lane.
   const bool nib = lut.nib_entries > 0;
   const size_t table = nib && lut.nib_shared ? lut.nib_entries * 4 : 0;
   const size_t class_max[4] = {nib ? table + 8 * 1024 : 40 * 1024, nib ? table + 32 * 1024 : 100 * 1024,

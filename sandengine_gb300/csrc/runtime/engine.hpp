@@ -101,8 +101,8 @@ struct World {
   // (the world's state) unchanged, for tuning trials.
   Status launch_tiles(int f0, int k, const TileVariant* v, bool commit = true, const EditParams* edits = nullptr,
                       int nedits = 0);
-  // Times every tile variant on this world (without changing it) and keeps the fastest
-  // multi-frame and one-frame variants.  *best_k gets the chosen frames per launch.
+  // Times the tile variants for this world on it (without changing it) and keeps the best
+  // multi-frame and one-frame variants: the fastest, 4-bit shapes weighed by their halo cells.  *best_k gets the chosen frames per launch.
   Status autotune(int reps, int* best_k);
   EditParams edit_params;  // the edit list of the current step's first launch (copied at launch)
   int default_k() const;
