@@ -394,9 +394,6 @@ Status World::step(int nframes, const se_modification* mods, int nmods) {
     vmulti = fused ? fused : vone;
   }
   const int kdef = steps_per_launch > 0 ? steps_per_launch : vmulti->kmax;
-  // a call's last frames, fewer than its launches take: a shape of few frames where one is meant for
-  // the world (tile_variants), unless the caller has chosen the tile
-  const bool few = steps_per_launch == 0 && !tile_asked && rs->lut_shape().nib_entries > 0;
   if (light[0]) {  // one frame at a time, each followed by the light pass
     for (int i = 0; i < nframes; ++i) {
       const int f = frame + 1 + i;
@@ -427,7 +424,9 @@ Status World::step(int nframes, const se_modification* mods, int nmods) {
     }
     const int k = std::min(kdef, nframes - i);
     const TileVariant* v = k == 1 ? vone : vmulti;
-    if (few && k > 1 && k < kdef) {
+    if (k > 1 && k < kdef && steps_per_launch == 0 && !tile_asked && rs->lut_shape().nib_entries) {
+      // a call's last frames, fewer than its launches take: a shape of few frames where one is meant for
+      // the world (tile_variants), unless the caller has chosen the tile
       const TileVariant* t = pick_variant(k, rs->lut_shape(), (long long)W * H);
       if (t->kmax < 8) v = t;
     }
